@@ -13,51 +13,50 @@
 
 namespace epx {
 
-constexpr int kMoeTileRows = 128;     // rows of one expert-sorted tile
+constexpr int kMoeTileRows = 128;     // granularity of the workspace bound below
 constexpr int kMoeGateUpTile = 128;   // intermediate columns produced by one GEMM-1 tile
 constexpr int kMoeDownTile = 256;     // hidden columns produced by one GEMM-2 tile
 
 struct MoeSizes {
-  long long max_sorted_rows;   // upper bound of expert-sorted rows incl. tile padding
-  int max_tiles;               // upper bound of 128-row tiles
+  long long max_sorted_rows;   // workspace rows: every local pair plus one tile of slack per expert
+  int max_tiles;               // the same in tiles of `tile_rows`
 };
 
 // CPU-known bounds for `rows` received rows, `topk` slots per row and `experts` local experts.
-// `tile_rows` is 128, or 256 when the GEMMs run on CTA pairs.
 MoeSizes moe_sizes(long long rows, int topk, int experts, int tile_rows = kMoeTileRows);
+// Entries of the token-tile list for `max_sorted_rows` sorted rows.
+long long moe_token_tiles(long long max_sorted_rows, int experts);
 
-// Groups the (row, slot) pairs of this rank's experts by expert into 128-row tiles.
-//   sorted_row   int32 [max_sorted_rows]  source row of every sorted position, -1 = padding
-//   sorted_scale f32   [max_sorted_rows]  routing weight of the pair, 0 for padding
-//   entry_pos    int32 [rows * topk]      sorted position of the pair, -1 when not local
-//   tile_expert  int32 [max_tiles]        local expert of every tile
+// Packs the (row, slot) pairs of this rank's experts by expert (no padding between experts) and
+// cuts every expert's rows into token tiles.
+//   sorted_row   int32 [max_sorted_rows]  source row of every sorted position
+//   sorted_scale f32   [max_sorted_rows]  routing weight of the pair
+//   entry_pos    int32 [rows * topk]      sorted position of the pair, -1 when not local (rows below *valid_count)
+//   tiles        int32 [moe_token_tiles][4]  {expert, first sorted row, rows, 0}, 16-byte aligned
 //   counters     int32 [2]                {tiles in use, sorted rows in use}
 //   error_flag   int32 [1]                set to 2 when max_sorted_rows was too small (pairs are dropped)
 cudaError_t launch_moe_align(const long long* local_ids, const float* weights, const int* valid_count, int rows,
-                             int topk, int experts, long long max_sorted_rows, int max_tiles, int* sorted_row,
-                             float* sorted_scale, int* entry_pos, int* tile_expert, int* counters,
-                             int* error_flag, int tile_rows, cudaStream_t stream);
+                             int topk, int experts, long long max_sorted_rows, int* sorted_row, float* sorted_scale,
+                             int* entry_pos, int* tiles, int* counters, int* error_flag, cudaStream_t stream);
 
-// sorted_x[pos] = hidden[sorted_row[pos]] (zero rows for padding) for the tiles in use.
-cudaError_t launch_moe_gather(const void* hidden, const int* sorted_row, const int* counters, void* sorted_x,
-                              long long max_sorted_rows, int hidden_size, cudaStream_t stream);
+// sorted_x[entry_pos[row, slot]] = hidden[row] for every local slot of the rows below *valid_count.
+cudaError_t launch_moe_scatter(const void* hidden, const int* entry_pos, const int* valid_count, void* sorted_x,
+                               int rows, int topk, int hidden_size, cudaStream_t stream);
 
 // GEMM 1: act[pos, :] = silu(x W1_e) * (x W3_e).  w13 is [experts, 2 * inter, hidden] (gate rows
 // first, then up rows), K-major. GEMM 2: y[pos, :] = (act W2_e) * sorted_scale[pos], w2 is
-// [experts, hidden, inter]. Shapes: hidden % 256 == 0, inter % 128 == 0. `pair` runs the GEMM on
-// clusters of two CTAs (tcgen05 cta_group::2, 256-row tiles: align with tile_rows = 256).
-// With `gather_rows` (= the align step's sorted_row, 16-byte aligned), `sorted_x` is the UNSORTED
-// activation matrix [gather_height, hidden]: the kernel's TMA producer gathers the rows of every
-// tile itself (four rows per copy) and no gather launch or sorted copy of the activations is needed.
+// [experts, hidden, inter]. Shapes: hidden % 256 == 0, inter % 128 == 0. `rows` is the same bound
+// that was given to the align step. With `gather_rows` (= the align step's sorted_row), `sorted_x`
+// is the UNSORTED activation matrix [gather_height, hidden]: the kernel's TMA producer gathers the
+// rows of every tile itself (four rows per copy) and no scatter launch or sorted copy is needed.
 cudaError_t launch_moe_gemm_gate_up(const void* sorted_x, const void* w13, void* act, const int* counters,
-                                    const int* tile_expert, int* error_flag, long long max_sorted_rows,
-                                    int experts, int hidden_size, int inter_size, int sms, bool pair,
-                                    cudaStream_t stream, const int* gather_rows = nullptr,
-                                    long long gather_height = 0);
+                                    const int* tiles, int* error_flag, long long rows, long long max_sorted_rows,
+                                    int experts, int hidden_size, int inter_size, int sms, cudaStream_t stream,
+                                    const int* gather_rows = nullptr, long long gather_height = 0);
 cudaError_t launch_moe_gemm_down(const void* act, const void* w2, void* y, const float* sorted_scale,
-                                 const int* counters, const int* tile_expert, int* error_flag,
+                                 const int* counters, const int* tiles, int* error_flag, long long rows,
                                  long long max_sorted_rows, int experts, int hidden_size, int inter_size, int sms,
-                                 bool pair, cudaStream_t stream);
+                                 cudaStream_t stream);
 
 // partial[row] = bf16(sum over slots, in slot order, of float(y[entry_pos[row, slot]])) for rows
 // below *valid_count.

@@ -1,29 +1,33 @@
-// Grouped SwiGLU expert GEMM for sm_100a: tcgen05.mma with TMEM accumulators, operands
-// staged in shared memory by TMA, one elected thread issuing the MMAs.
+// Grouped SwiGLU expert GEMM for sm_100a: tcgen05.mma on CTA pairs with TMEM accumulators,
+// operands staged in shared memory by TMA, one elected thread issuing the MMAs.
 //
 // The reference ships no expert GEMM: its adapter calls a framework's Triton kernel
 // around count-aware helper kernels (ep_xpress/adapters/sglang_valid.py:13-255). This
 // file is the hand-written replacement for that whole runner:
 //
-//   align      received (row, slot) pairs whose expert lives on this rank are grouped by
-//              expert into 128-row tiles bounded by the DEVICE valid_count (the job of
-//              sglang_valid.py:13-161);
-//   gather     activation rows are permuted into that expert-sorted order;
-//   GEMM 1     act = silu(x W1_e) * (x W3_e): gate and up columns of one output tile are
-//              accumulated side by side in TMEM (128 x 256 FP32) and fused in the epilogue
-//              (the framework needs a separate activation kernel,
-//              adapters/sglang/sglang-v0.5.21.patch:281-330);
+//   align      received (row, slot) pairs whose expert lives on this rank are packed by
+//              expert, bounded by the DEVICE valid_count (the job of
+//              sglang_valid.py:13-161), and every expert's rows are cut into token tiles;
+//   scatter    activation rows are copied into that expert-sorted order;
+//   GEMM 1     act = silu(x W1_e) * (x W3_e): gate and up rows of the weights sit in one
+//              tile, the epilogue pairs them up (the framework needs a separate activation
+//              kernel, adapters/sglang/sglang-v0.5.21.patch:281-330);
 //   GEMM 2     y = (act W2_e) * routing weight, rounded to BF16 per (row, slot);
 //   slot sum   partial[row] = bf16(sum over the row's local slots, in slot order, FP32) -
 //              the definition of a rank's partial (sglang_valid.py:206-222).
 //
-// Kernel structure (both GEMMs): persistent CTAs of 192 threads. Warp 0 elects one thread
-// that drives TMA loads into a 4-stage ring of 128B-swizzled K-major tiles; warp 1 elects
-// one thread that issues tcgen05.mma (M 128, N 256, K 16) and commits stage releases and
-// accumulator hand-offs to mbarriers; warps 2-5 are the epilogue, each owning the 32 TMEM
-// lanes of its quadrant. Two accumulator buffers (2 x 256 TMEM columns) let the epilogue of
-// one tile overlap the main loop of the next. Every wait is bounded and ends in an error
-// flag, after which TMEM is still released.
+// Which operand is M: the WEIGHTS. tcgen05 fixes M (256 rows on a CTA pair) but takes any
+// N = 16, 32, ... 256, and the number of tokens an expert got is the ragged dimension. With
+// tokens as N a tile costs what its tokens cost: no row is padded beyond the next multiple of
+// 16, so 32 experts with 32 tokens each stream their weights once instead of multiplying
+// 256-row tiles that are 7/8 padding, and expert segments are packed without gaps.
+// Measured (hidden 7168, inter 2048, 32 experts; tokens as 256-row M tiles -> tokens as N; us of
+// GEMM 1 + GEMM 2): 16 tokens per expert 366 + 186 -> 280 + 146 (6.4-6.7 TB/s of weights: HBM
+// bound), 1024 tokens 1285 + 676 -> 1290 + 650 (tensor bound,
+// nothing to pad). Hidden 2048, inter 768, 128 experts x 64 tokens: 294 + 110 -> 148 + 74.
+//
+// All launches of the runner are chained by programmatic dependent launch: a kernel's prologue
+// (barriers, TMEM, descriptors) and the dispatch of its CTAs overlap the tail of the one before.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,15 +38,16 @@
 namespace epx {
 namespace {
 
-constexpr int kTileM = 128;
-constexpr int kTileN = 256;
 constexpr int kTileK = 64;                 // 64 BF16 = one 128-byte swizzle row
-constexpr int kGemmStages = 4;
-constexpr int kABytes = kTileM * kTileK * 2;
-constexpr int kBBytes = kTileN * kTileK * 2;
-constexpr int kStageBytesGemm = kABytes + kBBytes;
+constexpr int kTileM = 256;                // weight rows of a CTA pair's tile (128 per CTA)
+constexpr int kMaxTileN = 256;             // tokens of a tile
+constexpr int kABytes = 128 * kTileK * 2;  // one CTA's weight rows of a k-step
+constexpr int kMaxStages = 12;
+constexpr int kRingBytes = 7 * (kABytes + kMaxTileN / 2 * kTileK * 2);   // 224 KB: seven stages of the widest tile
+constexpr size_t kGemmSmemBytes = kRingBytes + 1024;                      // + alignment of the swizzled tiles
 constexpr int kGemmThreads = 192;
 constexpr int kAccumColumns = 256;
+constexpr int kNMaps = 5;                  // boxes of 8, 16, 32, 64 and 128 token rows
 constexpr unsigned long long kGemmWaitNs = 2000000000ull;   // bound of every pipeline wait: 2 s
 
 // ---- PTX wrappers ----------------------------------------------------------------------
@@ -51,50 +56,11 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
   return pred != 0;
 }
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_address(bar)) : "memory");
-}
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
   return mbarrier_wait_bounded(bar, parity, kGemmWaitNs);
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(smem_address(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_address(bar)) : "memory");
-}
-// Four rows of a row-major matrix (any four row indices) x one 64-column box, written to `dst`
-// as four consecutive 128-byte rows; the tensor map has a box of {64, 1}. A row index at or
-// beyond the matrix height reads zeros. No fan-out: the copy lands in this CTA only.
-__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, int x, int r0, int r1, int r2, int r3,
-                                            unsigned long long* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-      ::"r"(smem_address(dst)), "l"(map), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(smem_address(bar))
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc(unsigned* smem_result, unsigned columns) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-               ::"r"(smem_address(smem_result)), "r"(columns) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(unsigned address, unsigned columns) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(address), "r"(columns) : "memory");
-}
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc,
-                                          unsigned idesc, unsigned accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// Arrives on `bar` once every MMA issued so far by this thread has finished.
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-               ::"r"(smem_address(bar)) : "memory");
-}
 __device__ __forceinline__ void tmem_load_32(unsigned taddr, unsigned (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -122,225 +88,6 @@ __device__ __forceinline__ constexpr unsigned instruction_descriptor(int m, int 
 }
 
 
-// ---- the grouped GEMM kernel -------------------------------------------------------------------
-struct GemmParams {
-  const int* num_m_tiles;        // device: 128-row tiles in use (depends on routing)
-  const int* tile_expert;        // device: [max tiles] local expert of each tile
-  const float* row_scale;        // kMode 1: routing weight of every sorted row
-  void* out;                     // bf16 [padded rows, out_columns]
-  int* error_flag;               // set to 1 when a bounded wait gave up
-  int k_steps;                   // K / 64
-  int n_tiles;                   // output column tiles per row tile
-  int out_columns;               // row pitch of `out` in elements
-  int b_rows_per_expert;         // rows of the weight matrix that belong to one expert
-  int up_row_offset;             // kMode 0: row distance between gate and up projections
-  const int* gather_rows;        // null, or [padded rows]: source row of every sorted position (-1: padding);
-                                 // the A operand is then gathered from the unsorted matrix behind map_a
-  int gather_height;             // rows of that matrix; an index at or above it reads zeros
-};
-
-// Row indices of lane `lane`'s four rows of the 128-row block that starts at `first`.
-__device__ __forceinline__ int4 gather_indices(const GemmParams& p, long long first, int lane) {
-  int4 rows = *reinterpret_cast<const int4*>(p.gather_rows + first + 4 * lane);
-  if (rows.x < 0) rows.x = p.gather_height;
-  if (rows.y < 0) rows.y = p.gather_height;
-  if (rows.z < 0) rows.z = p.gather_height;
-  if (rows.w < 0) rows.w = p.gather_height;
-  return rows;
-}
-
-// kMode 0: B tile = [128 gate rows; 128 up rows], epilogue silu(gate) * up -> 128 columns.
-// kMode 1: B tile = 256 rows, epilogue acc * row_scale -> 256 columns.
-template <int kMode>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const GemmParams p) {
-  extern __shared__ __align__(1024) unsigned char gemm_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
-  __shared__ unsigned long long full_bar[kGemmStages], empty_bar[kGemmStages];
-  __shared__ unsigned long long acc_full[2], acc_empty[2];
-  __shared__ unsigned tmem_base_slot;
-  __shared__ volatile int failed;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kGemmStages; ++s) {
-      mbarrier_init(full_bar + s, 1);
-      mbarrier_init(empty_bar + s, 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbarrier_init(acc_full + b, 1);
-      mbarrier_init(acc_empty + b, 4);          // one arrival per epilogue warp
-    }
-    failed = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
-  }
-  if (warp == 1) tmem_alloc(&tmem_base_slot, 2 * kAccumColumns);
-  tcgen05_fence_before();
-  __syncthreads();
-  tcgen05_fence_after();
-  const unsigned tmem_base = tmem_base_slot;
-
-  const int m_tiles = *p.num_m_tiles;
-  const long long total_tiles = static_cast<long long>(m_tiles) * p.n_tiles;
-  constexpr int kOutTile = kMode == 0 ? kTileN / 2 : kTileN;
-
-  if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (p.gather_rows != nullptr) {
-      // Gathered A operand: the whole warp takes part, lane l fetches rows 4l..4l+3 of the tile
-      // with ONE gather copy per k-step straight from the unsorted activation matrix.
-      unsigned use = 0;
-      bool go = true;
-      for (long long tile = blockIdx.x; tile < total_tiles && go; tile += gridDim.x) {
-        const int m_tile = static_cast<int>(tile / p.n_tiles), n_tile = static_cast<int>(tile % p.n_tiles);
-        const int expert = p.tile_expert[m_tile];
-        const int b_row = expert * p.b_rows_per_expert + n_tile * kOutTile;
-        const int4 rows = gather_indices(p, static_cast<long long>(m_tile) * kTileM, lane);
-        for (int k = 0; k < p.k_steps && go; ++k, ++use) {
-          const int s = use % kGemmStages;
-          unsigned char* a_dst = smem + static_cast<size_t>(s) * kStageBytesGemm;
-          unsigned char* b_dst = a_dst + kABytes;
-          int ok = 1;
-          if (lane == 0) {
-            ok = !failed && mbar_wait(empty_bar + s, ((use / kGemmStages) & 1u) ^ 1u) ? 1 : 0;
-            if (ok) mbarrier_arrive_expect_tx(full_bar + s, kStageBytesGemm);
-            else failed = 1;
-          }
-          go = __shfl_sync(0xffffffffu, ok, 0) != 0;
-          if (!go) break;
-          tma_gather4(a_dst + lane * 512, &map_a, k * kTileK, rows.x, rows.y, rows.z, rows.w, full_bar + s);
-          if (lane == 0) {
-            if (kMode == 0) {
-              tma_load_2d(b_dst, &map_b, k * kTileK, b_row, full_bar + s);
-              tma_load_2d(b_dst + kBBytes / 2, &map_b, k * kTileK, b_row + p.up_row_offset, full_bar + s);
-            } else {
-              tma_load_2d(b_dst, &map_b, k * kTileK, b_row, full_bar + s);
-            }
-          }
-        }
-      }
-    } else if (elect_one()) {
-      unsigned use = 0;
-      for (long long tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
-        const int m_tile = static_cast<int>(tile / p.n_tiles), n_tile = static_cast<int>(tile % p.n_tiles);
-        const int expert = p.tile_expert[m_tile];
-        const int b_row = expert * p.b_rows_per_expert + n_tile * kOutTile;
-        for (int k = 0; k < p.k_steps; ++k, ++use) {
-          const int s = use % kGemmStages;
-          if (!mbar_wait(empty_bar + s, ((use / kGemmStages) & 1u) ^ 1u)) { failed = 1; break; }
-          unsigned char* a_dst = smem + static_cast<size_t>(s) * kStageBytesGemm;
-          unsigned char* b_dst = a_dst + kABytes;
-          mbarrier_arrive_expect_tx(full_bar + s, kStageBytesGemm);
-          tma_load_2d(a_dst, &map_a, k * kTileK, m_tile * kTileM, full_bar + s);
-          if (kMode == 0) {
-            tma_load_2d(b_dst, &map_b, k * kTileK, b_row, full_bar + s);
-            tma_load_2d(b_dst + kBBytes / 2, &map_b, k * kTileK, b_row + p.up_row_offset, full_bar + s);
-          } else {
-            tma_load_2d(b_dst, &map_b, k * kTileK, b_row, full_bar + s);
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (elect_one()) {
-      constexpr unsigned idesc = instruction_descriptor(kTileM, kTileN);
-      unsigned use = 0, local_tile = 0;
-      for (long long tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++local_tile) {
-        const unsigned buffer = local_tile & 1u;
-        if (!mbar_wait(acc_empty + buffer, ((local_tile >> 1) & 1u) ^ 1u)) { failed = 1; break; }
-        tcgen05_fence_after();
-        const unsigned tmem_d = tmem_base + buffer * kAccumColumns;
-        for (int k = 0; k < p.k_steps; ++k, ++use) {
-          const int s = use % kGemmStages;
-          if (!mbar_wait(full_bar + s, (use / kGemmStages) & 1u)) { failed = 1; break; }
-          tcgen05_fence_after();
-          const unsigned char* a_tile = smem + static_cast<size_t>(s) * kStageBytesGemm;
-          const unsigned long long a_desc = smem_descriptor(a_tile);
-          const unsigned long long b_desc = smem_descriptor(a_tile + kABytes);
-#pragma unroll
-          for (int kk = 0; kk < kTileK / 16; ++kk)   // 16 BF16 = 32 bytes = 2 descriptor units per step
-            umma_bf16(tmem_d, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (k | kk) != 0 ? 1u : 0u);
-          umma_commit(empty_bar + s);                 // stage reusable when these MMAs retire
-        }
-        if (failed) break;
-        umma_commit(acc_full + buffer);               // accumulator complete
-      }
-    }
-  } else {
-    // ---------------- epilogue: warps 2..5, TMEM lane quadrant = warp % 4 ----------------
-    const int quadrant = warp & 3;
-    const int row_in_tile = quadrant * 32 + lane;
-    unsigned local_tile = 0;
-    for (long long tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++local_tile) {
-      const int m_tile = static_cast<int>(tile / p.n_tiles), n_tile = static_cast<int>(tile % p.n_tiles);
-      const unsigned buffer = local_tile & 1u;
-      const bool ok = mbar_wait(acc_full + buffer, (local_tile >> 1) & 1u);
-      if (!__all_sync(0xffffffffu, ok)) { failed = 1; break; }
-      tcgen05_fence_after();
-      const unsigned taddr = tmem_base + buffer * kAccumColumns + (static_cast<unsigned>(quadrant * 32) << 16);
-      const long long row = static_cast<long long>(m_tile) * kTileM + row_in_tile;
-      __nv_bfloat16* out_row = reinterpret_cast<__nv_bfloat16*>(p.out) + row * p.out_columns +
-                               static_cast<long long>(n_tile) * kOutTile;
-      const float scale = kMode == 1 ? p.row_scale[row] : 1.f;
-#pragma unroll 1
-      for (int chunk = 0; chunk < kOutTile / 32; ++chunk) {
-        unsigned first[32];
-        unsigned second[32];
-        tmem_load_32(taddr + chunk * 32, first);
-        if (kMode == 0) tmem_load_32(taddr + kTileN / 2 + chunk * 32, second);
-        tmem_load_wait();
-        unsigned packed[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float lo, hi;
-          if (kMode == 0) {
-            const float g0 = __uint_as_float(first[2 * i]), g1 = __uint_as_float(first[2 * i + 1]);
-            lo = (g0 / (1.f + __expf(-g0))) * __uint_as_float(second[2 * i]);
-            hi = (g1 / (1.f + __expf(-g1))) * __uint_as_float(second[2 * i + 1]);
-          } else {
-            lo = __uint_as_float(first[2 * i]) * scale;
-            hi = __uint_as_float(first[2 * i + 1]) * scale;
-          }
-          packed[i] = pack_bf16x2(lo, hi);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(out_row + chunk * 32);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-      }
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty + buffer);
-    }
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tcgen05_fence_after();
-    tmem_dealloc(tmem_base, 2 * kAccumColumns);
-  }
-  if (threadIdx.x == 0 && failed) atomicExch(p.error_flag, 1);
-}
-
-
-// ---- the same GEMM on CTA pairs (thread-block clusters of two, tcgen05 cta_group::2) ------------
-// One 128 x 256 tile per SM needs 48 KB of operands per k-step; at full tensor rate that is
-// more L2 bandwidth x latency than four stages of shared memory can keep in flight. A pair
-// of CTAs computes a 256 x 256 tile instead: each CTA stages its own 128 rows of A and HALF
-// of the B tile (32 KB per k-step, six stages), the leader CTA's elected thread issues
-// tcgen05.mma.cta_group::2 which reads both CTAs' shared memory and writes each CTA's half
-// of the accumulator into that CTA's own TMEM, and both CTAs run their own epilogue. Both
-// producers complete their TMA loads on the LEADER's full barrier; the leader commits stage
-// releases and accumulator hand-offs to both CTAs' barriers. No load fans out to more than
-// one CTA: each CTA fetches exactly the bytes it keeps.
-constexpr int kPairStages = 6;
-constexpr int kPairBBytes = kBBytes / 2;
-constexpr int kPairStageBytes = kABytes + kPairBBytes;
-constexpr size_t kPairSmemBytes = static_cast<size_t>(kPairStages) * kPairStageBytes + 1024;
 
 __device__ __forceinline__ unsigned cluster_ctarank() {
   unsigned r;
@@ -364,13 +111,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_address(dst)), "l"(map), "r"(x), "r"(y), "r"(bar_cluster) : "memory");
 }
-__device__ __forceinline__ void tma_gather4_pair(void* dst, const CUtensorMap* map, int x, int r0, int r1, int r2, int r3,
-                                                 unsigned bar_cluster) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 "
-      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-      ::"r"(smem_address(dst)), "l"(map), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar_cluster) : "memory");
-}
 __device__ __forceinline__ void tmem_alloc_pair(unsigned* smem_result, unsigned columns) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                ::"r"(smem_address(smem_result)), "r"(columns) : "memory");
@@ -386,27 +126,96 @@ __device__ __forceinline__ void umma_bf16_pair(unsigned tmem_d, unsigned long lo
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_commit_pair(unsigned bar_cluster) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster)
-               : "memory");
+
+// The weights of GEMM 1 as a five-dimensional box {64 k, 16 rows, gate/up, 4 blocks, expert}: 128
+// rows of shared memory that alternate 16 gate rows with the 16 up rows of the same columns.
+__device__ __forceinline__ void tma_load_5d_pair(void* dst, const CUtensorMap* map, int x, int block, int expert,
+                                                 unsigned bar_cluster) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %3, %4, %5}], [%6];"
+      ::"r"(smem_address(dst)), "l"(map), "r"(x), "r"(0), "r"(block), "r"(expert), "r"(bar_cluster) : "memory");
+}
+// Four rows of a row-major matrix (any four row indices) x one 64-column box, written to `dst`
+// as four consecutive 128-byte rows; the tensor map has a box of {64, 1}. A row index at or
+// beyond the matrix height reads zeros. No fan-out: the copy lands in this CTA only.
+__device__ __forceinline__ void tma_gather4_pair(void* dst, const CUtensorMap* map, int x, int r0, int r1, int r2, int r3,
+                                                 unsigned bar_cluster) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+      ::"r"(smem_address(dst)), "l"(map), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar_cluster) : "memory");
+}
+// Arrives on the barrier at this offset in BOTH CTAs of the pair once every MMA issued so far by
+// this thread has finished.
+__device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_address(bar)), "h"(static_cast<unsigned short>(3)) : "memory");
+}
+// Programmatic dependent launch: the next kernel of the chain may start its prologue / everything
+// the previous kernel wrote is visible from here on. (Both return at once in an ordinary launch.)
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ---- the grouped GEMM kernel -------------------------------------------------------------------
+struct GemmParams {
+  const int* counters;           // device: {token tiles in use, sorted rows in use}
+  const int4* tiles;             // device: {expert, first sorted row, rows, -} of every token tile
+  const float* row_scale;        // kMode 1: routing weight of every sorted row
+  void* out;                     // bf16 [sorted rows, out_columns]
+  int* error_flag;               // set to 1 when a bounded wait gave up
+  int k_steps;                   // K / 64
+  int m_tiles;                   // 256-row weight tiles of one expert
+  int out_columns;               // row pitch of `out` in elements
+  int b_rows;                    // token rows a stage has room for in one CTA (half of the widest tile)
+  int stages;
+  const int* gather_rows;        // null, or [sorted rows]: source row of every sorted position; the token operand
+                                 // is then gathered from the unsorted matrix behind maps.b[0]
+  int gather_height;             // rows of that matrix; an index at or above it reads zeros
+};
+struct GemmMaps {
+  CUtensorMap a;
+  CUtensorMap b[kNMaps];         // the token matrix with boxes of 8 << i rows
+};
+
+// Index of the smallest box that holds `half` token rows (a multiple of 8).
+__device__ __forceinline__ int box_index(int half) {
+  return half <= 8 ? 0 : (half <= 16 ? 1 : (half <= 32 ? 2 : (half <= 64 ? 3 : 4)));
 }
 
+// One 256 x N tile per CTA pair (a cluster of two), N = the tile's tokens rounded up to 16. Each
+// CTA stages its own 128 weight rows and HALF of the tokens; the leader CTA's elected thread
+// issues tcgen05.mma.cta_group::2, which reads both CTAs' shared memory and writes each CTA's 128
+// accumulator rows into that CTA's own TMEM, and both CTAs run their own epilogue. Both producers
+// complete their TMA loads on the LEADER's full barrier; the leader's commits release stages and
+// hand over accumulators in both CTAs. No load fans out to more than one CTA.
+//
+// Persistent: pair c takes tiles c, c + pairs, ... in (token tile, weight tile) order, so the
+// pairs that run together share one expert's tokens and, for experts with several token tiles,
+// its weights in L2. Warp 0 feeds the ring, warp 1 issues MMAs, warps 2-5 drain the accumulators
+// (two buffers of 256 TMEM columns, so the epilogue of one tile overlaps the next main loop).
+// Every wait is bounded and ends in an error flag, after which TMEM is still released.
+//
+// kMode 0: 256 weight rows = 128 gate and 128 up rows of the same columns, interleaved by 16, so
+//          a gate row and its up row are 16 lanes apart in one warp: epilogue silu(gate) * up.
+// kMode 1: 256 rows of W2, epilogue acc * row_scale.
 template <int kMode>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                         const GemmParams p) {
+grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
   extern __shared__ __align__(1024) unsigned char gemm_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) &
                                                          ~static_cast<uintptr_t>(1023));
-  __shared__ unsigned long long full_bar[kPairStages], empty_bar[kPairStages];
+  __shared__ unsigned long long full_bar[kMaxStages], empty_bar[kMaxStages];
   __shared__ unsigned long long acc_full[2], acc_empty[2];
   __shared__ unsigned tmem_base_slot;
   __shared__ volatile int failed;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned rank = cluster_ctarank();           // 0 = leader
+  const int stages = p.stages;
+  const int stage_bytes = kABytes + p.b_rows * kTileK * 2;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kPairStages; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbarrier_init(full_bar + s, 1);                // leader's: one arrive.expect_tx + both CTAs' bytes
       mbarrier_init(empty_bar + s, 1);               // one commit from the leader per use
     }
@@ -425,128 +234,142 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   tcgen05_fence_after();
   const unsigned tmem_base = tmem_base_slot;
 
-  const int m_tiles = *p.num_m_tiles;                // 256-row tiles
-  const long long total_tiles = static_cast<long long>(m_tiles) * p.n_tiles;
-  const long long cluster_id = blockIdx.x / 2, clusters = gridDim.x / 2;
-  constexpr int kOutTile = kMode == 0 ? kTileN / 2 : kTileN;
-  constexpr int kPairM = 2 * kTileM;
+  wait_for_previous();
+  launch_dependents();
+  const int total = p.counters[0] * p.m_tiles;
+  const int pair_id = blockIdx.x / 2, pairs = gridDim.x / 2;
+
+  auto load_weights = [&](unsigned char* dst, int k, int expert, int mt, unsigned leader_full) {
+    if (kMode == 0) tma_load_5d_pair(dst, &maps.a, k * kTileK, mt * 8 + static_cast<int>(rank) * 4, expert, leader_full);
+    else tma_load_2d_pair(dst, &maps.a, k * kTileK, (expert * p.m_tiles + mt) * kTileM + static_cast<int>(rank) * 128, leader_full);
+  };
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
+    // One ELECTED thread issues: the same loop under `if (lane == 0)` cost the tensor pipe a fifth of
+    // its cycles (hidden 7168, inter 2048, 32 experts x 1024 tokens: 1431 + 746 us against 1290 + 646),
+    // because without elect.sync the compiler cannot keep the copies' operands in uniform registers.
+    int s = 0;
+    unsigned parity = 1u;                            // of the stage's empty barrier: the first round passes at once
     if (p.gather_rows != nullptr) {
-      // Gathered A operand (see the single-CTA kernel): each CTA gathers its own 128 rows.
-      unsigned use = 0;
+      // Gathered tokens: the whole warp takes part, every lane fetches four rows per k-step.
       bool go = true;
-      for (long long tile = cluster_id; tile < total_tiles && go; tile += clusters) {
-        const int m_tile = static_cast<int>(tile / p.n_tiles), n_tile = static_cast<int>(tile % p.n_tiles);
-        const int expert = p.tile_expert[m_tile];
-        const int b_row = expert * p.b_rows_per_expert + n_tile * kOutTile +
-                          (kMode == 0 ? static_cast<int>(rank) * p.up_row_offset : static_cast<int>(rank) * (kTileN / 2));
-        const int4 rows = gather_indices(p, static_cast<long long>(m_tile) * kPairM + static_cast<long long>(rank) * kTileM, lane);
-        for (int k = 0; k < p.k_steps && go; ++k, ++use) {
-          const int s = use % kPairStages;
-          unsigned char* a_dst = smem + static_cast<size_t>(s) * kPairStageBytes;
+      for (int item = pair_id; item < total && go; item += pairs) {
+        const int tt = item / p.m_tiles, mt = item - tt * p.m_tiles;
+        const int4 tile = p.tiles[tt];
+        const int half = ((tile.z + 15) & ~15) / 2;
+        const bool fetch = 4 * lane < half;
+        const int first = static_cast<int>(rank) * half + 4 * lane;
+        int rows[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          rows[i] = fetch && first + i < tile.z ? p.gather_rows[tile.y + first + i] : p.gather_height;
+        for (int k = 0; k < p.k_steps; ++k) {
+          unsigned char* a_dst = smem + static_cast<size_t>(s) * stage_bytes;
           const unsigned leader_full = peer_smem_address(full_bar + s, 0);
-          int ok = 1;
-          if (lane == 0) {
-            ok = !failed && mbar_wait(empty_bar + s, ((use / kPairStages) & 1u) ^ 1u) ? 1 : 0;
-            if (!ok) failed = 1;
-            else if (rank == 0) mbarrier_arrive_expect_tx(full_bar + s, 2 * kPairStageBytes);
+          const bool ok = !failed && mbar_wait(empty_bar + s, parity);
+          go = __all_sync(0xffffffffu, ok);
+          if (!go) { failed = 1; break; }
+          if (elect_one()) {
+            if (rank == 0) mbarrier_arrive_expect_tx(full_bar + s, 2u * (kABytes + half * kTileK * 2));
+            load_weights(a_dst, k, tile.x, mt, leader_full);
           }
-          go = __shfl_sync(0xffffffffu, ok, 0) != 0;
-          if (!go) break;
-          tma_gather4_pair(a_dst + lane * 512, &map_a, k * kTileK, rows.x, rows.y, rows.z, rows.w, leader_full);
-          if (lane == 0) tma_load_2d_pair(a_dst + kABytes, &map_b, k * kTileK, b_row, leader_full);
+          __syncwarp();
+          if (fetch) tma_gather4_pair(a_dst + kABytes + lane * 512, maps.b, k * kTileK, rows[0], rows[1], rows[2], rows[3], leader_full);
+          if (++s == stages) { s = 0; parity ^= 1u; }
         }
       }
     } else if (elect_one()) {
-      unsigned use = 0;
-      for (long long tile = cluster_id; tile < total_tiles && !failed; tile += clusters) {
-        const int m_tile = static_cast<int>(tile / p.n_tiles), n_tile = static_cast<int>(tile % p.n_tiles);
-        const int expert = p.tile_expert[m_tile];
-        // Mode 0: the leader keeps the gate rows, its peer the up rows. Mode 1: halves of the tile.
-        const int b_row = expert * p.b_rows_per_expert + n_tile * kOutTile +
-                          (kMode == 0 ? static_cast<int>(rank) * p.up_row_offset : static_cast<int>(rank) * (kTileN / 2));
-        for (int k = 0; k < p.k_steps; ++k, ++use) {
-          const int s = use % kPairStages;
-          if (!mbar_wait(empty_bar + s, ((use / kPairStages) & 1u) ^ 1u)) { failed = 1; break; }
-          unsigned char* a_dst = smem + static_cast<size_t>(s) * kPairStageBytes;
+      for (int item = pair_id; item < total && !failed; item += pairs) {
+        const int tt = item / p.m_tiles, mt = item - tt * p.m_tiles;
+        const int4 tile = p.tiles[tt];
+        const int half = ((tile.z + 15) & ~15) / 2;
+        const int which = box_index(half);
+        const CUtensorMap* map_b = maps.b + which;
+        const unsigned tx = 2u * (kABytes + (8u << which) * kTileK * 2);
+        const int b_row = tile.y + static_cast<int>(rank) * half;
+        for (int k = 0; k < p.k_steps; ++k) {
+          unsigned char* a_dst = smem + static_cast<size_t>(s) * stage_bytes;
           const unsigned leader_full = peer_smem_address(full_bar + s, 0);
-          if (rank == 0) mbarrier_arrive_expect_tx(full_bar + s, 2 * kPairStageBytes);
-          tma_load_2d_pair(a_dst, &map_a, k * kTileK, m_tile * kPairM + static_cast<int>(rank) * kTileM, leader_full);
-          tma_load_2d_pair(a_dst + kABytes, &map_b, k * kTileK, b_row, leader_full);
+          if (!mbar_wait(empty_bar + s, parity)) { failed = 1; break; }
+          if (rank == 0) mbarrier_arrive_expect_tx(full_bar + s, tx);
+          load_weights(a_dst, k, tile.x, mt, leader_full);
+          tma_load_2d_pair(a_dst + kABytes, map_b, k * kTileK, b_row, leader_full);
+          if (++s == stages) { s = 0; parity ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader only) ----------------
     if (rank == 0 && elect_one()) {
-      constexpr unsigned idesc = instruction_descriptor(kPairM, kTileN);
-      unsigned use = 0, local_tile = 0;
-      for (long long tile = cluster_id; tile < total_tiles && !failed; tile += clusters, ++local_tile) {
+      int s = 0;
+      unsigned parity = 0u, local_tile = 0;
+      for (int item = pair_id; item < total && !failed; item += pairs, ++local_tile) {
+        const int n = (p.tiles[item / p.m_tiles].z + 15) & ~15;
+        const unsigned idesc = instruction_descriptor(kTileM, n);
         const unsigned buffer = local_tile & 1u;
         if (!mbar_wait(acc_empty + buffer, ((local_tile >> 1) & 1u) ^ 1u)) { failed = 1; break; }
         tcgen05_fence_after();
         const unsigned tmem_d = tmem_base + buffer * kAccumColumns;
-        for (int k = 0; k < p.k_steps; ++k, ++use) {
-          const int s = use % kPairStages;
-          if (!mbar_wait(full_bar + s, (use / kPairStages) & 1u)) { failed = 1; break; }
+        for (int k = 0; k < p.k_steps; ++k) {
+          if (!mbar_wait(full_bar + s, parity)) { failed = 1; break; }
           tcgen05_fence_after();
-          const unsigned char* a_tile = smem + static_cast<size_t>(s) * kPairStageBytes;
+          const unsigned char* a_tile = smem + static_cast<size_t>(s) * stage_bytes;
           const unsigned long long a_desc = smem_descriptor(a_tile);
           const unsigned long long b_desc = smem_descriptor(a_tile + kABytes);
 #pragma unroll
-          for (int kk = 0; kk < kTileK / 16; ++kk)
+          for (int kk = 0; kk < kTileK / 16; ++kk)   // 16 BF16 = 32 bytes = 2 descriptor units per step
             umma_bf16_pair(tmem_d, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (k | kk) != 0 ? 1u : 0u);
-          umma_commit_pair(peer_smem_address(empty_bar + s, 0));     // both CTAs may refill the stage
-          umma_commit_pair(peer_smem_address(empty_bar + s, 1));
+          umma_commit_pair(empty_bar + s);           // both CTAs may refill the stage
+          if (++s == stages) { s = 0; parity ^= 1u; }
         }
         if (failed) break;
-        umma_commit_pair(peer_smem_address(acc_full + buffer, 0));   // both epilogues may read
-        umma_commit_pair(peer_smem_address(acc_full + buffer, 1));
+        umma_commit_pair(acc_full + buffer);         // both epilogues may read
       }
     }
   } else {
-    // ---------------- epilogue (both CTAs, own 128 rows) ----------------
+    // ---------------- epilogue (both CTAs, own 128 weight rows) ----------------
+    // TMEM lane = weight row (output column), TMEM column = token.
     const int quadrant = warp & 3;
-    const int row_in_tile = static_cast<int>(rank) * kTileM + quadrant * 32 + lane;
     unsigned local_tile = 0;
-    for (long long tile = cluster_id; tile < total_tiles; tile += clusters, ++local_tile) {
-      const int m_tile = static_cast<int>(tile / p.n_tiles), n_tile = static_cast<int>(tile % p.n_tiles);
+    for (int item = pair_id; item < total; item += pairs, ++local_tile) {
+      const int tt = item / p.m_tiles, mt = item - tt * p.m_tiles;
+      const int4 tile = p.tiles[tt];
       const unsigned buffer = local_tile & 1u;
       const bool ok = mbar_wait(acc_full + buffer, (local_tile >> 1) & 1u);
       if (!__all_sync(0xffffffffu, ok)) { failed = 1; break; }
       tcgen05_fence_after();
       const unsigned taddr = tmem_base + buffer * kAccumColumns + (static_cast<unsigned>(quadrant * 32) << 16);
-      const long long row = static_cast<long long>(m_tile) * kPairM + row_in_tile;
-      __nv_bfloat16* out_row = reinterpret_cast<__nv_bfloat16*>(p.out) + row * p.out_columns +
-                               static_cast<long long>(n_tile) * kOutTile;
-      const float scale = kMode == 1 ? p.row_scale[row] : 1.f;
+      const int upper = lane >> 4;                   // kMode 0: lanes 0-15 hold gate rows, 16-31 their up rows
+      const int column = kMode == 0 ? mt * 128 + static_cast<int>(rank) * 64 + quadrant * 16 + (lane & 15)
+                                    : mt * kTileM + static_cast<int>(rank) * 128 + quadrant * 32 + lane;
+      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(tile.y) * p.out_columns + column;
 #pragma unroll 1
-      for (int chunk = 0; chunk < kOutTile / 32; ++chunk) {
-        unsigned first[32];
-        unsigned second[32];
-        tmem_load_32(taddr + chunk * 32, first);
-        if (kMode == 0) tmem_load_32(taddr + kTileN / 2 + chunk * 32, second);
+      for (int c0 = 0; c0 < tile.z; c0 += 32) {
+        unsigned v[32];
+        tmem_load_32(taddr + c0, v);
         tmem_load_wait();
-        unsigned packed[16];
+        if (kMode == 0) {
+          // A lane pair (l, l + 16) holds gate and up of 32 tokens: the lower lane finishes the first
+          // sixteen of them, the upper lane the others.
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float lo, hi;
-          if (kMode == 0) {
-            const float g0 = __uint_as_float(first[2 * i]), g1 = __uint_as_float(first[2 * i + 1]);
-            lo = (g0 / (1.f + __expf(-g0))) * __uint_as_float(second[2 * i]);
-            hi = (g1 / (1.f + __expf(-g1))) * __uint_as_float(second[2 * i + 1]);
-          } else {
-            lo = __uint_as_float(first[2 * i]) * scale;
-            hi = __uint_as_float(first[2 * i + 1]) * scale;
+          for (int i = 0; i < 16; ++i) {
+            const float mine = __uint_as_float(upper ? v[16 + i] : v[i]);
+            const float theirs = __uint_as_float(__shfl_xor_sync(0xffffffffu, upper ? v[i] : v[16 + i], 16));
+            const float gate = upper ? theirs : mine, up = upper ? mine : theirs;
+            const int token = c0 + upper * 16 + i;
+            if (token < tile.z)
+              out[static_cast<long long>(token) * p.out_columns] = __float2bfloat16_rn((gate / (1.f + __expf(-gate))) * up);
           }
-          packed[i] = pack_bf16x2(lo, hi);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(out_row + chunk * 32);
+        } else {
+          const float scale = c0 + lane < tile.z ? p.row_scale[tile.y + c0 + lane] : 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+          for (int i = 0; i < 32; ++i) {
+            const float w = __shfl_sync(0xffffffffu, scale, i);
+            if (c0 + i < tile.z)
+              out[static_cast<long long>(c0 + i) * p.out_columns] = __float2bfloat16_rn(__uint_as_float(v[i]) * w);
+          }
+        }
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -563,136 +386,226 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (threadIdx.x == 0 && failed) atomicExch(p.error_flag, 1);
 }
 
-// ---- align / gather / slot-sum helper kernels ---------------------------------------------------
+// ---- align / scatter / slot-sum helper kernels ---------------------------------------------------
 constexpr int kAlignThreads = 1024;
 constexpr int kMaxLocalExperts = 1024;
+constexpr int kAlignClusterMax = 8;
 
-__global__ void __launch_bounds__(256) moe_fill_kernel(int* sorted_row, float* sorted_scale, long long sorted_rows,
-                                                       int* entry_pos, long long entries) {
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  const long long me = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  for (long long i = me; i < sorted_rows; i += stride) { sorted_row[i] = -1; sorted_scale[i] = 0.f; }
-  for (long long i = me; i < entries; i += stride) entry_pos[i] = -1;
+// Exclusive prefix sum over the CTA's 1024 threads (`warp_sums` is 32 words of shared memory).
+__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int upto = v;
+#pragma unroll
+  for (int step = 1; step < 32; step <<= 1) {
+    const int below = __shfl_up_sync(0xffffffffu, upto, step);
+    if (lane >= step) upto += below;
+  }
+  __syncthreads();
+  if (lane == 31) warp_sums[warp] = upto;
+  __syncthreads();
+  int base = 0;
+  for (int w = 0; w < warp; ++w) base += warp_sums[w];
+  return base + upto - v;
 }
 
-// One CTA: histogram per local expert, tile-padded prefix, scatter. Bounded by the device
-// valid_count, never by a host-side count.
+// A chain of memory and barrier latencies, not bandwidth. One cluster of 1-8 CTAs packs the local (row, slot) pairs by expert: every CTA counts its share
+// of the pairs per expert in shared memory (the counting atomic also ranks the pair inside the
+// CTA), the CTAs read each other's counts through distributed shared memory, every CTA derives
+// the same prefix sums, and the second pass writes each pair to expert base + CTA base + rank.
+// Bounded by the device valid_count, never by a host-side count; order inside an expert is free
+// (a row's results do not depend on it). 2048 pairs per CTA is where a second CTA starts to pay for
+// the cluster barriers. 32768 pairs of 4096 rows: 11 us, against 64 us for one CTA that counted,
+// then counted again while scattering, plus 2.6 us for a launch that preset its outputs; 1024
+// pairs: 5.5 us against 8.1 + 1.3.
 __global__ void __launch_bounds__(kAlignThreads) moe_align_kernel(const long long* __restrict__ local_ids,
                                                                   const float* __restrict__ weights,
                                                                   const int* __restrict__ valid_count, int rows,
-                                                                  int topk, int experts, long long max_sorted_rows,
-                                                                  int max_tiles, int tile, int* sorted_row, float* sorted_scale,
-                                                                  int* entry_pos, int* tile_expert, int* counters,
+                                                                  int topk, int experts, int max_sorted_rows,
+                                                                  int tile_cap, int* sorted_row, float* sorted_scale,
+                                                                  int* entry_pos, int4* tiles, int* counters,
                                                                   int* error_flag) {
   __shared__ int s_count[kMaxLocalExperts];
-  __shared__ int s_offset[kMaxLocalExperts];
-  const int valid = min(*valid_count, rows);
-  const long long pairs = static_cast<long long>(valid) * topk;
-  for (int e = threadIdx.x; e < experts; e += kAlignThreads) s_count[e] = 0;
+  __shared__ int s_base[kMaxLocalExperts];
+  __shared__ int s_scan[32];
+  unsigned cta, ctas;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+  const int tid = threadIdx.x;
+  s_count[tid] = 0;
   __syncthreads();
-  for (long long i = threadIdx.x; i < pairs; i += kAlignThreads) {
-    const long long id = local_ids[i];
-    if (id >= 0 && id < experts) atomicAdd(&s_count[id], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int offset = 0, tiles = 0;
-    for (int e = 0; e < experts; ++e) {
-      const int padded = (s_count[e] + tile - 1) / tile * tile;
-      s_offset[e] = offset;
-      for (int t = 0; t < padded / tile && tiles < max_tiles; ++t) tile_expert[tiles++] = e;
-      offset += padded;
+  wait_for_previous();
+  launch_dependents();
+  const int pairs = min(*valid_count, rows) * topk;
+  const int step = static_cast<int>(ctas) * kAlignThreads;
+  constexpr int kBatch = 4;                          // independent loads in flight per thread
+  for (int first = static_cast<int>(cta) * kAlignThreads + tid; first < pairs; first += kBatch * step) {
+    long long id[kBatch];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) id[b] = first + b * step < pairs ? local_ids[first + b * step] : -1;
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      if (first + b * step < pairs)
+        entry_pos[first + b * step] = id[b] >= 0 && id[b] < experts ? atomicAdd(&s_count[id[b]], 1) : -1;
     }
-    if (offset > max_sorted_rows) {           // the caller's bound on local pairs was too small
-      atomicExch(error_flag, 2);
-      offset = static_cast<int>(max_sorted_rows);
+  }
+  cluster_sync();
+  // Thread e: rows of expert e in the whole cluster and in the CTAs before this one.
+  int mine = 0, before = 0;
+  if (tid < experts) {
+    for (unsigned c = 0; c < ctas; ++c) {
+      unsigned v;
+      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_smem_address(s_count + tid, c)) : "memory");
+      mine += static_cast<int>(v);
+      if (c < cta) before += static_cast<int>(v);
     }
-    counters[0] = tiles < offset / tile ? tiles : offset / tile;
-    counters[1] = offset;
+  }
+  const int offset = block_exclusive_scan(mine, s_scan);
+  s_base[tid] = offset + before;
+  if (cta == 0) {
+    // Token tiles: an expert's rows in equal parts of at most `tile_cap`, a multiple of 16 each.
+    const int usable = max(0, min(mine, max_sorted_rows - offset));
+    const int parts = (usable + tile_cap - 1) / tile_cap;
+    const int part = parts > 0 ? ((usable + parts - 1) / parts + 15) / 16 * 16 : 0;
+    const int at = block_exclusive_scan(parts, s_scan);
+    for (int i = 0; i < parts; ++i)
+      tiles[at + i] = make_int4(tid, offset + i * part, min(part, usable - i * part), 0);
+    if (tid == kAlignThreads - 1) {
+      counters[0] = at + parts;
+      counters[1] = min(offset + mine, max_sorted_rows);
+      if (offset + mine > max_sorted_rows) atomicExch(error_flag, 2);   // the caller's bound on local pairs was too small
+    }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < experts; e += kAlignThreads) s_count[e] = 0;
-  __syncthreads();
-  for (long long i = threadIdx.x; i < pairs; i += kAlignThreads) {
-    const long long id = local_ids[i];
-    if (id < 0 || id >= experts) continue;
-    const long long pos = s_offset[id] + atomicAdd(&s_count[id], 1);
-    if (pos >= max_sorted_rows) continue;
-    sorted_row[pos] = static_cast<int>(i / topk);
-    sorted_scale[pos] = weights[i];
-    entry_pos[i] = static_cast<int>(pos);
+  for (int first = static_cast<int>(cta) * kAlignThreads + tid; first < pairs; first += kBatch * step) {
+    int at[kBatch];
+    long long id[kBatch];
+    float w[kBatch];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int i = first + b * step;
+      at[b] = i < pairs ? entry_pos[i] : -1;
+      id[b] = i < pairs ? local_ids[i] : -1;
+      w[b] = i < pairs ? weights[i] : 0.f;
+    }
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int i = first + b * step;
+      if (at[b] < 0) continue;
+      const int pos = s_base[id[b]] + at[b];
+      if (pos < max_sorted_rows) {
+        sorted_row[pos] = i / topk;
+        sorted_scale[pos] = w[b];
+      }
+      entry_pos[i] = pos < max_sorted_rows ? pos : -1;
+    }
   }
+  cluster_sync();                                    // nobody leaves while a peer may still read its counts
 }
 
-__global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* __restrict__ hidden, const int* __restrict__ sorted_row,
-                                                         const int* __restrict__ counters, uint4* __restrict__ sorted_x,
-                                                         long long max_sorted_rows, int vecs_per_row) {
-  const long long used = min(static_cast<long long>(counters[1]), max_sorted_rows);
+// Both row movers work on units of 128 16-byte vectors (2 KB of a row, four vectors per lane), one
+// unit per warp and pass: a single decode row is spread over several warps, and four independent
+// 16-byte accesses per lane and slot cover the memory latency of a large batch.
+constexpr int kUnitVecs = 128;
+__device__ __forceinline__ int units_per_row(int vecs_per_row) { return (vecs_per_row + kUnitVecs - 1) / kUnitVecs; }
+
+// sorted_x[entry_pos[row, slot]] = hidden[row] for every local slot: a row is read ONCE and stored to
+// every expert it goes to. HBM bound: 4096 rows x 8 slots x 14 KB (529 MB) in 91 us = 5.8 TB/s;
+// gathering per sorted position read each row eight times and wrote padding: 149 us.
+__global__ void __launch_bounds__(256) moe_scatter_kernel(const uint4* __restrict__ hidden, const int* __restrict__ entry_pos,
+                                                          const int* __restrict__ valid_count, uint4* __restrict__ sorted_x,
+                                                          int rows, int topk, int vecs_per_row) {
+  wait_for_previous();
+  launch_dependents();
   const int lane = threadIdx.x & 31;
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x / 32);
-  for (long long pos = static_cast<long long>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5); pos < used;
-       pos += warps) {
-    const int row = sorted_row[pos];
-    uint4* dst = sorted_x + pos * vecs_per_row;
-    const uint4* src = hidden + static_cast<long long>(row < 0 ? 0 : row) * vecs_per_row;
-    for (int base = lane; base < vecs_per_row; base += 128) {
-      uint4 v[4];
+  const unsigned units = units_per_row(vecs_per_row);
+  const unsigned items = min(*valid_count, rows) * units;
+  const unsigned warps = gridDim.x * (blockDim.x / 32);
+  for (unsigned item = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); item < items; item += warps) {
+    const unsigned row = item / units;
+    const int base = static_cast<int>(item - row * units) * kUnitVecs + lane;
+    const int* positions = entry_pos + static_cast<long long>(row) * topk;
+    const uint4* src = hidden + static_cast<long long>(row) * vecs_per_row;
+    uint4 v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (base + u * 32 < vecs_per_row) v[u] = row < 0 ? make_uint4(0, 0, 0, 0) : src[base + u * 32];
+    for (int u = 0; u < 4; ++u)
+      if (base + u * 32 < vecs_per_row) v[u] = src[base + u * 32];
+    for (int k0 = 0; k0 < topk; k0 += 32) {
+      const int mine = k0 + lane < topk ? positions[k0 + lane] : -1;
+      for (unsigned local = __ballot_sync(0xffffffffu, mine >= 0); local != 0; local &= local - 1) {
+        const int pos = __shfl_sync(0xffffffffu, mine, __ffs(local) - 1);
+        uint4* dst = sorted_x + static_cast<long long>(pos) * vecs_per_row;
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (base + u * 32 < vecs_per_row) dst[base + u * 32] = v[u];
+        for (int u = 0; u < 4; ++u)
+          if (base + u * 32 < vecs_per_row) dst[base + u * 32] = v[u];
+      }
     }
   }
 }
 
+// partial[row] = the row's local slots of y added in slot order; two slots' loads are in flight at a
+// time. A unit per warp instead of a row per warp: one decode row of eight slots 51 -> 5 us, 128 rows
+// 68 -> 7 us (one warp walked 56 dependent loads); large batches are HBM bound either way (4096 rows
+// x 8 slots, 529 MB: about 110 us).
 __global__ void __launch_bounds__(256) moe_slot_sum_kernel(const uint4* __restrict__ y, const int* __restrict__ entry_pos,
                                                            const int* __restrict__ valid_count, uint4* __restrict__ partial,
                                                            int rows, int topk, int vecs_per_row) {
-  const int valid = min(*valid_count, rows);
+  wait_for_previous();
+  launch_dependents();
   const int lane = threadIdx.x & 31;
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x / 32);
-  for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5); row < valid;
-       row += warps) {
-    // Lane k holds the sorted position of slot k (fetched once per row, not once per chunk).
-    const int slots = min(topk, 32);
-    const int my_pos = lane < slots ? entry_pos[row * topk + lane] : -1;
-    for (int start = 0; start < vecs_per_row; start += 64) {          // warp-uniform; two chunks per lane in flight
-      const int base = start + lane;
-      float acc[2][8];
+  const unsigned units = units_per_row(vecs_per_row);
+  const unsigned items = min(*valid_count, rows) * units;
+  const unsigned warps = gridDim.x * (blockDim.x / 32);
+  for (unsigned item = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); item < items; item += warps) {
+    const unsigned row = item / units;
+    const int base = static_cast<int>(item - row * units) * kUnitVecs + lane;
+    const int* positions = entry_pos + static_cast<long long>(row) * topk;
+    unsigned long long acc[4][4];
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
-      for (int k = 0; k < topk; ++k) {
-        const int pos = k < 32 ? __shfl_sync(0xffffffffu, my_pos, k) : entry_pos[row * topk + k];
-        if (pos < 0) continue;
+      for (int i = 0; i < 4; ++i) acc[u][i] = 0ull;
+    auto fetch = [&](uint4 (&v)[4], int pos) {
+      const uint4* src = y + static_cast<long long>(pos) * vecs_per_row;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int at = base + u * 32;
-          if (at < vecs_per_row) {
-            const uint4 v = y[static_cast<long long>(pos) * vecs_per_row + at];
-            const unsigned w[4] = {v.x, v.y, v.z, v.w};
+      for (int u = 0; u < 4; ++u)
+        if (base + u * 32 < vecs_per_row) v[u] = src[base + u * 32];
+    };
+    auto add = [&](const uint4 (&v)[4]) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              acc[u][2 * i] = __fadd_rn(acc[u][2 * i], __uint_as_float(w[i] << 16));
-              acc[u][2 * i + 1] = __fadd_rn(acc[u][2 * i + 1], __uint_as_float(w[i] & 0xffff0000u));
-            }
-          }
-        }
+      for (int u = 0; u < 4; ++u) {
+        acc[u][0] = add_f32x2(acc[u][0], bf16x2_to_f32x2(v[u].x));
+        acc[u][1] = add_f32x2(acc[u][1], bf16x2_to_f32x2(v[u].y));
+        acc[u][2] = add_f32x2(acc[u][2], bf16x2_to_f32x2(v[u].z));
+        acc[u][3] = add_f32x2(acc[u][3], bf16x2_to_f32x2(v[u].w));
       }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int at = base + u * 32;
-        if (at < vecs_per_row) {
-          unsigned out[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            out[i] = pack_bf16x2(acc[u][2 * i], acc[u][2 * i + 1]);
-          partial[row * vecs_per_row + at] = make_uint4(out[0], out[1], out[2], out[3]);
+    };
+    for (int k0 = 0; k0 < topk; k0 += 32) {
+      const int mine = k0 + lane < topk ? positions[k0 + lane] : -1;
+      unsigned local = __ballot_sync(0xffffffffu, mine >= 0);
+      while (local != 0) {
+        uint4 first[4] = {}, second[4] = {};
+        fetch(first, __shfl_sync(0xffffffffu, mine, __ffs(local) - 1));
+        local &= local - 1;
+        const bool two = local != 0;
+        if (two) {
+          fetch(second, __shfl_sync(0xffffffffu, mine, __ffs(local) - 1));
+          local &= local - 1;
         }
+        add(first);
+        if (two) add(second);
       }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (base + u * 32 >= vecs_per_row) continue;
+      unsigned out[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float lo, hi;
+        unpack_f32x2(acc[u][i], lo, hi);
+        out[i] = pack_bf16x2(lo, hi);
+      }
+      partial[static_cast<long long>(row) * vecs_per_row + base + u * 32] = make_uint4(out[0], out[1], out[2], out[3]);
     }
   }
 }
@@ -715,55 +628,65 @@ EncodeTiled encode_tiled() {
 }
 
 // Row-major BF16 matrix [rows, columns]; box = box_rows x 64 columns, 128-byte swizzle.
-cudaError_t make_map(CUtensorMap* map, const void* base, long long rows, long long columns, int box_rows) {
-  EncodeTiled encode = encode_tiled();
-  if (encode == nullptr) return cudaErrorNotSupported;
+bool make_map(CUtensorMap* map, const void* base, long long rows, long long columns, int box_rows) {
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(columns), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(columns) * 2};
   const cuuint32_t box[2] = {kTileK, static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t element_strides[2] = {1, 1};
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
-                            element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+  return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
+                        element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Same matrix addressed one row at a time (box 1 x 64 columns): the form gather copies need.
-cudaError_t make_gather_map(CUtensorMap* map, const void* base, long long rows, long long columns) {
-  return make_map(map, base, rows, columns, 1);
+// w13 [experts, gate/up, inter, hidden] as {hidden, 16 rows, gate/up, inter / 16, experts}; a box of
+// {64, 16, 2, 4, 1} is 128 shared-memory rows: 16 gate rows, their 16 up rows, the next 16 gate rows ...
+bool make_gate_up_map(CUtensorMap* map, const void* base, int experts, int inter, int hidden) {
+  const cuuint64_t row = static_cast<cuuint64_t>(hidden) * 2;
+  const cuuint64_t dims[5] = {static_cast<cuuint64_t>(hidden), 16, 2, static_cast<cuuint64_t>(inter / 16),
+                              static_cast<cuuint64_t>(experts)};
+  const cuuint64_t strides[4] = {row, row * inter, row * 16, row * inter * 2};
+  const cuuint32_t box[5] = {kTileK, 16, 2, 4, 1};
+  const cuuint32_t element_strides[5] = {1, 1, 1, 1, 1};
+  return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box,
+                        element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr size_t kGemmSmemBytes = static_cast<size_t>(kGemmStages) * kStageBytesGemm + 1024;
-
-template <int kMode>
-cudaError_t launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& params, int sms,
-                             cudaStream_t stream) {
-  cudaError_t err = cudaFuncSetAttribute(grouped_gemm_pair_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(kPairSmemBytes));
-  if (err != cudaSuccess) return err;
+// A launch of the runner's chain: programmatic dependent launch, so that the kernel's prologue
+// overlaps the tail of the one before it (every kernel of the chain waits before it touches data).
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), int ctas, int threads, int cluster, size_t smem,
+                           cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t config{};
-  config.gridDim = dim3(sms / 2 * 2, 1, 1);
-  config.blockDim = dim3(kGemmThreads, 1, 1);
-  config.dynamicSmemBytes = kPairSmemBytes;
+  config.gridDim = dim3(ctas, 1, 1);
+  config.blockDim = dim3(threads, 1, 1);
+  config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = 2;
-  attribute.val.clusterDim.y = 1;
-  attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, grouped_gemm_pair_kernel<kMode>, map_a, map_b, params);
+  cudaLaunchAttribute attributes[2]{};
+  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[0].val.programmaticStreamSerializationAllowed = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = cluster;
+  attributes[1].val.clusterDim.y = 1;
+  attributes[1].val.clusterDim.z = 1;
+  config.attrs = attributes;
+  config.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+// Ring geometry: small batches use narrow token boxes and more stages.
+void set_ring(GemmParams* params, int tile_cap) {
+  params->b_rows = tile_cap / 2;
+  const int stages = kRingBytes / (kABytes + params->b_rows * kTileK * 2);
+  params->stages = stages < kMaxStages ? stages : kMaxStages;
 }
 
 template <int kMode>
-cudaError_t launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& params, int sms,
-                        cudaStream_t stream) {
+cudaError_t launch_gemm(GemmMaps& maps, const GemmParams& params, int sms, cudaStream_t stream) {
   cudaError_t err = cudaFuncSetAttribute(grouped_gemm_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kGemmSmemBytes));
   if (err != cudaSuccess) return err;
-  grouped_gemm_kernel<kMode><<<sms, kGemmThreads, kGemmSmemBytes, stream>>>(map_a, map_b, params);
-  return cudaGetLastError();
+  return launch_chained(grouped_gemm_kernel<kMode>, sms / 2 * 2, kGemmThreads, 2, kGemmSmemBytes, stream, maps, params);
 }
 
 }  // namespace
@@ -777,91 +700,104 @@ MoeSizes moe_sizes(long long rows, int topk, int experts, int tile_rows) {
   return sizes;
 }
 
+// An expert gets at most one slot of every row (the router chooses without replacement; ids that
+// do repeat only cost more tiles), so `rows` bounds the widest useful tile.
+int moe_tile_cap(long long rows) {
+  int cap = 16;
+  while (cap < kMaxTileN && cap < rows) cap *= 2;
+  return cap;
+}
+long long moe_token_tiles(long long max_sorted_rows, int experts) { return max_sorted_rows / 16 + experts; }
+
 cudaError_t launch_moe_align(const long long* local_ids, const float* weights, const int* valid_count, int rows,
-                             int topk, int experts, long long max_sorted_rows, int max_tiles, int* sorted_row,
-                             float* sorted_scale, int* entry_pos, int* tile_expert, int* counters,
-                             int* error_flag, int tile_rows, cudaStream_t stream) {
-  if (experts > kMaxLocalExperts || (tile_rows != kTileM && tile_rows != 2 * kTileM)) return cudaErrorInvalidValue;
-  moe_fill_kernel<<<296, 256, 0, stream>>>(sorted_row, sorted_scale, max_sorted_rows, entry_pos,
-                                           static_cast<long long>(rows) * topk);
-  moe_align_kernel<<<1, kAlignThreads, 0, stream>>>(local_ids, weights, valid_count, rows, topk, experts,
-                                                    max_sorted_rows, max_tiles, tile_rows, sorted_row, sorted_scale,
-                                                    entry_pos, tile_expert, counters, error_flag);
-  return cudaGetLastError();
+                             int topk, int experts, long long max_sorted_rows, int* sorted_row,
+                             float* sorted_scale, int* entry_pos, int* tiles, int* counters,
+                             int* error_flag, cudaStream_t stream) {
+  const long long pairs = static_cast<long long>(rows) * topk;
+  if (experts > kMaxLocalExperts || pairs >= (1ll << 30) || max_sorted_rows >= (1ll << 30)) return cudaErrorInvalidValue;
+  int cluster = 1;
+  while (cluster < kAlignClusterMax && pairs > 2ll * kAlignThreads * cluster) cluster *= 2;
+  return launch_chained(moe_align_kernel, cluster, kAlignThreads, cluster, 0, stream, local_ids, weights, valid_count,
+                        rows, topk, experts, static_cast<int>(max_sorted_rows), moe_tile_cap(rows), sorted_row, sorted_scale, entry_pos,
+                        reinterpret_cast<int4*>(tiles), counters, error_flag);
 }
 
-cudaError_t launch_moe_gather(const void* hidden, const int* sorted_row, const int* counters, void* sorted_x,
-                              long long max_sorted_rows, int hidden_size, cudaStream_t stream) {
+// CTAs of a row mover: one warp per unit, at most eight CTAs of eight warps per SM.
+static int mover_ctas(long long rows, int hidden_size) {
+  const long long items = rows * ((hidden_size / 8 + kUnitVecs - 1) / kUnitVecs);
+  return items < 148 * 8 * 8 ? static_cast<int>((items + 7) / 8) : 148 * 8;
+}
+
+cudaError_t launch_moe_scatter(const void* hidden, const int* entry_pos, const int* valid_count, void* sorted_x,
+                               int rows, int topk, int hidden_size, cudaStream_t stream) {
   if (hidden_size % 8) return cudaErrorInvalidValue;
-  moe_gather_kernel<<<148 * 8, 256, 0, stream>>>(static_cast<const uint4*>(hidden), sorted_row, counters,
-                                                 static_cast<uint4*>(sorted_x), max_sorted_rows, hidden_size / 8);
-  return cudaGetLastError();
+  if (rows <= 0) return cudaSuccess;
+  return launch_chained(moe_scatter_kernel, mover_ctas(rows, hidden_size), 256, 1, 0, stream,
+                        static_cast<const uint4*>(hidden), entry_pos, valid_count, static_cast<uint4*>(sorted_x), rows,
+                        topk, hidden_size / 8);
 }
 
 cudaError_t launch_moe_gemm_gate_up(const void* sorted_x, const void* w13, void* act, const int* counters,
-                                    const int* tile_expert, int* error_flag, long long max_sorted_rows,
-                                    int experts, int hidden_size, int inter_size, int sms, bool pair,
-                                    cudaStream_t stream, const int* gather_rows, long long gather_height) {
+                                    const int* tiles, int* error_flag, long long rows, long long max_sorted_rows,
+                                    int experts, int hidden_size, int inter_size, int sms, cudaStream_t stream,
+                                    const int* gather_rows, long long gather_height) {
   if (hidden_size % kTileK || inter_size % kMoeGateUpTile) return cudaErrorInvalidValue;
-  if (gather_rows != nullptr && (gather_height <= 0 || gather_height >= (1ll << 31) ||
-                                 reinterpret_cast<uintptr_t>(gather_rows) % 16 != 0))
-    return cudaErrorInvalidValue;
-  CUtensorMap map_a, map_b;
-  // With `gather_rows`, `sorted_x` is the UNSORTED activation matrix [gather_height, hidden].
-  cudaError_t err = gather_rows != nullptr ? make_gather_map(&map_a, sorted_x, gather_height, hidden_size)
-                                           : make_map(&map_a, sorted_x, max_sorted_rows, hidden_size, kTileM);
-  if (err != cudaSuccess) return err;
-  err = make_map(&map_b, w13, static_cast<long long>(experts) * 2 * inter_size, hidden_size, kTileN / 2);
-  if (err != cudaSuccess) return err;
+  if (gather_rows != nullptr && (gather_height <= 0 || gather_height >= (1ll << 31))) return cudaErrorInvalidValue;
+  if (encode_tiled() == nullptr) return cudaErrorNotSupported;
+  GemmMaps maps{};
   GemmParams params{};
-  params.num_m_tiles = counters;
-  params.tile_expert = tile_expert;
+  set_ring(&params, moe_tile_cap(rows));
+  bool ok = make_gate_up_map(&maps.a, w13, experts, inter_size, hidden_size);
+  if (gather_rows != nullptr) {
+    ok = ok && make_map(&maps.b[0], sorted_x, gather_height, hidden_size, 1);   // gather copies take one-row boxes
+  } else {
+    for (int i = 0; i < kNMaps && (8 << i) <= params.b_rows; ++i)
+      ok = ok && make_map(&maps.b[i], sorted_x, max_sorted_rows, hidden_size, 8 << i);
+  }
+  if (!ok) return cudaErrorInvalidValue;
+  params.counters = counters;
+  params.tiles = reinterpret_cast<const int4*>(tiles);
   params.out = act;
   params.error_flag = error_flag;
   params.k_steps = hidden_size / kTileK;
-  params.n_tiles = inter_size / kMoeGateUpTile;
+  params.m_tiles = inter_size / kMoeGateUpTile;
   params.out_columns = inter_size;
-  params.b_rows_per_expert = 2 * inter_size;
-  params.up_row_offset = inter_size;
   params.gather_rows = gather_rows;
   params.gather_height = static_cast<int>(gather_height);
-  return pair ? launch_gemm_pair<0>(map_a, map_b, params, sms, stream)
-              : launch_gemm<0>(map_a, map_b, params, sms, stream);
+  return launch_gemm<0>(maps, params, sms, stream);
 }
 
 cudaError_t launch_moe_gemm_down(const void* act, const void* w2, void* y, const float* sorted_scale,
-                                 const int* counters, const int* tile_expert, int* error_flag,
+                                 const int* counters, const int* tiles, int* error_flag, long long rows,
                                  long long max_sorted_rows, int experts, int hidden_size, int inter_size, int sms,
-                                 bool pair, cudaStream_t stream) {
+                                 cudaStream_t stream) {
   if (inter_size % kTileK || hidden_size % kMoeDownTile) return cudaErrorInvalidValue;
-  CUtensorMap map_a, map_b;
-  cudaError_t err = make_map(&map_a, act, max_sorted_rows, inter_size, kTileM);
-  if (err != cudaSuccess) return err;
-  err = make_map(&map_b, w2, static_cast<long long>(experts) * hidden_size, inter_size, pair ? kTileN / 2 : kTileN);
-  if (err != cudaSuccess) return err;
+  if (encode_tiled() == nullptr) return cudaErrorNotSupported;
+  GemmMaps maps{};
   GemmParams params{};
-  params.num_m_tiles = counters;
-  params.tile_expert = tile_expert;
+  set_ring(&params, moe_tile_cap(rows));
+  bool ok = make_map(&maps.a, w2, static_cast<long long>(experts) * hidden_size, inter_size, 128);
+  for (int i = 0; i < kNMaps && (8 << i) <= params.b_rows; ++i)
+    ok = ok && make_map(&maps.b[i], act, max_sorted_rows, inter_size, 8 << i);
+  if (!ok) return cudaErrorInvalidValue;
+  params.counters = counters;
+  params.tiles = reinterpret_cast<const int4*>(tiles);
   params.row_scale = sorted_scale;
   params.out = y;
   params.error_flag = error_flag;
   params.k_steps = inter_size / kTileK;
-  params.n_tiles = hidden_size / kMoeDownTile;
+  params.m_tiles = hidden_size / kMoeDownTile;
   params.out_columns = hidden_size;
-  params.b_rows_per_expert = hidden_size;
-  params.up_row_offset = 0;
-  return pair ? launch_gemm_pair<1>(map_a, map_b, params, sms, stream)
-              : launch_gemm<1>(map_a, map_b, params, sms, stream);
+  return launch_gemm<1>(maps, params, sms, stream);
 }
 
 cudaError_t launch_moe_slot_sum(const void* y, const int* entry_pos, const int* valid_count, void* partial,
                                 int rows, int topk, int hidden_size, cudaStream_t stream) {
   if (hidden_size % 8) return cudaErrorInvalidValue;
   if (rows <= 0) return cudaSuccess;
-  const int ctas = rows < 148 * 8 * 8 ? (rows + 7) / 8 : 148 * 8;
-  moe_slot_sum_kernel<<<ctas, 256, 0, stream>>>(static_cast<const uint4*>(y), entry_pos, valid_count,
-                                                static_cast<uint4*>(partial), rows, topk, hidden_size / 8);
-  return cudaGetLastError();
+  return launch_chained(moe_slot_sum_kernel, mover_ctas(rows, hidden_size), 256, 1, 0, stream,
+                        static_cast<const uint4*>(y), entry_pos, valid_count, static_cast<uint4*>(partial), rows, topk,
+                        hidden_size / 8);
 }
 
 }  // namespace epx

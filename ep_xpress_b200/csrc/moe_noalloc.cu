@@ -16,6 +16,7 @@ constexpr long long kSortedRows = 1024;
 constexpr long long kMaxPairs = 8192;
 constexpr int kMaxHidden = 1024;
 constexpr int kMaxInter = 512;
+constexpr long long kMaxTiles = kSortedRows / 16 + kSortedRows / 128;   // moe_token_tiles() at the limits: each expert takes >= 128 rows
 constexpr int kMaxDevices = 64;
 
 constexpr size_t align256(size_t v) { return (v + 255) / 256 * 256; }
@@ -24,8 +25,8 @@ constexpr size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 constexpr size_t kOffSortedRow = 0;                                                    // int32 [kSortedRows]
 constexpr size_t kOffSortedScale = kOffSortedRow + align256(kSortedRows * 4);          // f32   [kSortedRows]
 constexpr size_t kOffEntryPos = kOffSortedScale + align256(kSortedRows * 4);           // int32 [kMaxPairs]
-constexpr size_t kOffTileExpert = kOffEntryPos + align256(kMaxPairs * 4);              // int32 [kSortedRows / 128]
-constexpr size_t kOffCounters = kOffTileExpert + align256(kSortedRows / 128 * 4);      // int32 [2] + error flag
+constexpr size_t kOffTiles = kOffEntryPos + align256(kMaxPairs * 4);                   // int32 [kMaxTiles][4]
+constexpr size_t kOffCounters = kOffTiles + align256(kMaxTiles * 16);                  // int32 [2] + error flag
 constexpr size_t kOffSortedX = kOffCounters + 256;                                     // bf16 [kSortedRows, kMaxHidden]
 constexpr size_t kOffAct = kOffSortedX + align256(kSortedRows * kMaxHidden * 2);       // bf16 [kSortedRows, kMaxInter]
 constexpr size_t kOffY = kOffAct + align256(kSortedRows * kMaxInter * 2);              // bf16 [kSortedRows, kMaxHidden]
@@ -115,7 +116,7 @@ extern "C" int epx_moe_forward_noalloc(const void* hidden, const long long* loca
   int* sorted_row = reinterpret_cast<int*>(base + kOffSortedRow);
   float* sorted_scale = reinterpret_cast<float*>(base + kOffSortedScale);
   int* entry_pos = reinterpret_cast<int*>(base + kOffEntryPos);
-  int* tile_expert = reinterpret_cast<int*>(base + kOffTileExpert);
+  int* tiles = reinterpret_cast<int*>(base + kOffTiles);
   int* counters = reinterpret_cast<int*>(base + kOffCounters);
   int* error_flag = counters + 2;
   void* sorted_x = base + kOffSortedX;
@@ -128,17 +129,16 @@ extern "C" int epx_moe_forward_noalloc(const void* hidden, const long long* loca
   if (err != cudaSuccess) return fail(err);
   if (rows == 0) return EPX_NOALLOC_OK;
   const long long sorted_rows = sizes.max_sorted_rows;   // <= kSortedRows, a multiple of 128
-  err = epx::launch_moe_align(local_ids, weights, valid_count, rows, topk, experts, sorted_rows, sizes.max_tiles,
-                              sorted_row, sorted_scale, entry_pos, tile_expert, counters, error_flag,
-                              epx::kMoeTileRows, stream);
+  err = epx::launch_moe_align(local_ids, weights, valid_count, rows, topk, experts, sorted_rows, sorted_row,
+                              sorted_scale, entry_pos, tiles, counters, error_flag, stream);
   if (err != cudaSuccess) return fail(err);
-  err = epx::launch_moe_gather(hidden, sorted_row, counters, sorted_x, sorted_rows, hidden_size, stream);
+  err = epx::launch_moe_scatter(hidden, entry_pos, valid_count, sorted_x, rows, topk, hidden_size, stream);
   if (err != cudaSuccess) return fail(err);
-  err = epx::launch_moe_gemm_gate_up(sorted_x, w13, act, counters, tile_expert, error_flag, sorted_rows, experts,
-                                     hidden_size, inter_size, state->sms, false, stream);
+  err = epx::launch_moe_gemm_gate_up(sorted_x, w13, act, counters, tiles, error_flag, rows, sorted_rows, experts,
+                                     hidden_size, inter_size, state->sms, stream);
   if (err != cudaSuccess) return fail(err);
-  err = epx::launch_moe_gemm_down(act, w2, y, sorted_scale, counters, tile_expert, error_flag, sorted_rows, experts,
-                                  hidden_size, inter_size, state->sms, false, stream);
+  err = epx::launch_moe_gemm_down(act, w2, y, sorted_scale, counters, tiles, error_flag, rows, sorted_rows, experts,
+                                  hidden_size, inter_size, state->sms, stream);
   if (err != cudaSuccess) return fail(err);
   err = epx::launch_moe_slot_sum(y, entry_pos, valid_count, partial, rows, topk, hidden_size, stream);
   if (err != cudaSuccess) return fail(err);

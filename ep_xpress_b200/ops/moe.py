@@ -27,12 +27,13 @@ class GroupedSwiGLU:
 
         ``gather_loads=True``: the first GEMM's TMA producer gathers the activation rows of every
         expert tile straight from the dispatch batch (``tile::gather4``, four rows per copy), so
-        no gather launch and no expert-sorted copy of the activations exist. Bit-identical, but
-        opt-in: a 128-row operand tile then takes 32 copies of 512 bytes per k-step instead of
+        no scatter launch and no expert-sorted copy of the activations exist. Bit-identical, but
+        opt-in: 128 token rows then take 32 copies of 512 bytes per k-step instead of
         one 16 KB box, and the copy engine's issue rate, not the tensor pipe, bounds the GEMM
         (measured at hidden 7168 / inter 2048, 2 GPUs, 4096 tokens per rank: 7.4 ms against
-        3.7 ms with the gather kernel, whose cost is 0.15 ms).
+        3.7 ms with a copy kernel, whose cost is 0.1 to 0.15 ms).
 
+        ``pair_ctas`` is accepted either way: every GEMM runs on clusters of two CTAs.
 
         The default is the worst case (every slot of every row is local). A tighter,
         CPU-known bound saves workspace; exceeding it is reported by :meth:`check`,
@@ -49,7 +50,7 @@ class GroupedSwiGLU:
         self.native = _native_loader.load()
         self.w13, self.w2 = w13.contiguous(), w2.contiguous()
         self.experts, self.hidden, self.inter, self.topk, self.max_rows = experts, hidden, inter, topk, max_rows
-        self.pair_ctas = bool(pair_ctas)        # GEMMs on clusters of two CTAs (256-row tiles)
+        self.pair_ctas = bool(pair_ctas)        # accepted either way: the GEMMs always run on clusters of two CTAs
         tile = self.native.MOE_TILE_ROWS * (2 if self.pair_ctas else 1)
         worst_rows, _ = self.native.moe_sizes(max_rows, topk, experts, tile)
         if max_local_pairs is None:
@@ -61,7 +62,7 @@ class GroupedSwiGLU:
         self.sorted_row = torch.empty(sorted_rows, dtype=torch.int32, device=device)
         self.sorted_scale = torch.empty(sorted_rows, dtype=torch.float32, device=device)
         self.entry_pos = torch.empty(max_rows * topk, dtype=torch.int32, device=device)
-        self.tile_expert = torch.zeros(sorted_rows // tile, dtype=torch.int32, device=device)
+        self.tiles = torch.zeros((self.native.moe_token_tiles(sorted_rows, experts), 4), dtype=torch.int32, device=device)
         self.counters = torch.zeros(2, dtype=torch.int32, device=device)
         self.error_flag = torch.zeros(1, dtype=torch.int32, device=device)
         self.gather_loads = bool(gather_loads)
@@ -69,7 +70,7 @@ class GroupedSwiGLU:
                                                                    device=device)
         self.act = torch.empty((sorted_rows, inter), dtype=torch.bfloat16, device=device)
         self.y = torch.empty((sorted_rows, hidden), dtype=torch.bfloat16, device=device)
-        self.kernel_launches_per_forward = 5 if self.gather_loads else 6
+        self.kernel_launches_per_forward = 4 if self.gather_loads else 5
 
     def forward(self, hidden, local_ids, weights, valid_count, out=None, stream=None):
         rows = hidden.shape[0]
@@ -81,8 +82,8 @@ class GroupedSwiGLU:
         if self.gather_loads and (rows == 0 or hidden.data_ptr() % 16):
             raise ValueError("gathered loads need a non-empty, 16-byte aligned activation matrix")
         self.native.moe_forward(hidden, local_ids, weights, valid_count, self.w13, self.w2, out, self.sorted_row,
-                                self.sorted_scale, self.entry_pos, self.tile_expert, self.counters, self.error_flag,
-                                self.sorted_x, self.act, self.y, stream.cuda_stream, self.pair_ctas)
+                                self.sorted_scale, self.entry_pos, self.tiles, self.counters, self.error_flag,
+                                self.sorted_x, self.act, self.y, stream.cuda_stream)
         return out
 
     __call__ = forward

@@ -100,6 +100,35 @@ def test_cta_pairs_match_fp32_reference_and_single_cta_path(rows, topk, experts,
     assert torch.equal(other[:valid], out[:valid])     # same accumulation order per output row
 
 
+@pytest.mark.parametrize("counts,pad", [
+    ([0, 1, 15, 16, 17, 31, 33, 0], 3),               # one narrow tile each, experts without rows
+    ([63, 65, 127, 128, 129, 2], 0),                  # every token-box size
+    ([255, 256, 257, 0, 511, 513], 40),               # one, two and three token tiles per expert
+    ([2047], 1), ([1, 2047], 0), ([4090, 7], 0),      # one, two and four CTAs in the align step
+    ([1], 0),
+])
+@pytest.mark.parametrize("gather_loads", [True, False])
+def test_token_tile_edges_match_fp32_reference(counts, pad, gather_loads):
+    """Rows per expert at the edges of the token tiles; rows of one expert are spread over the batch."""
+    hidden, inter = 256, 128
+    g = torch.Generator().manual_seed(sum(counts))
+    experts = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    valid = len(experts)
+    ids = torch.full((valid + pad, 2), -1, dtype=torch.int64)
+    ids[torch.arange(valid), torch.randint(0, 2, (valid,), generator=g)] = experts[torch.randperm(valid, generator=g)]
+    x = (torch.randn((valid + pad, hidden), generator=g) * 0.5).to(torch.bfloat16)
+    weights = torch.rand((valid + pad, 2), generator=g)
+    w13 = (torch.randn((len(counts), 2 * inter, hidden), generator=g) * 0.05).to(torch.bfloat16)
+    w2 = (torch.randn((len(counts), hidden, inter), generator=g) * 0.05).to(torch.bfloat16)
+    x, ids, weights, w13, w2 = (t.cuda() for t in (x, ids, weights, w13, w2))
+    runner = GroupedSwiGLU(w13, w2, max_rows=valid + pad, topk=2, gather_loads=gather_loads)
+    out = torch.full((valid + pad, hidden), 7.0, dtype=torch.bfloat16, device="cuda")
+    runner(x, ids, weights, torch.tensor([valid], dtype=torch.int32, device="cuda"), out=out)
+    runner.check()
+    assert_elementwise_close(out[:valid], swiglu_reference(x, ids, weights, valid, w13, w2)[:valid])
+    assert (out[valid:] == 7.0).all()
+
+
 def test_pair_bound_overflow_is_reported():
     x, ids, weights, count, w13, w2 = make_case(512, 4, 2, 256, 128, 512, seed=3, local_fraction=1.0)
     runner = GroupedSwiGLU(w13, w2, max_rows=512, topk=4, max_local_pairs=128)
