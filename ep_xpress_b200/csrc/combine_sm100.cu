@@ -1044,87 +1044,93 @@ combine_kernel(const __grid_constant__ CombineArgs args) {
 // the same rounding helpers as the general reduce (0 + x in FP32, so -0 becomes +0 there too).
 // A pass like that is bound by memory latency, not by arithmetic: it wants many resident warps
 // with several 16-byte loads in flight each, not one 640-thread CTA per SM with its stage rings.
-// So it is a plain launch of small CTAs, one warp per token at a time. Epoch, sample ring and
-// error reporting are those of the general kernel; profiled operations use the general kernel.
+// So it is a plain launch of small CTAs; a warp takes units of 2 KB of a row, four 16-byte loads per
+// lane. (A warp per row left all but a tenth of the chip idle at decode sizes.) The context and the
+// slot layout come as kernel parameters and are at hand before the wait for the previous kernel.
+// Epoch, sample ring and error reporting are those of the general kernel; profiled operations use the
+// general kernel.
 constexpr int kLoneThreads = 256;
-constexpr int kLoneUnroll = 8;
+constexpr int kLoneUnroll = 4;
 constexpr int kLoneSms = 148;
 constexpr int kLoneMaxCtas = kLoneSms * 8;
 
-__global__ void __launch_bounds__(kLoneThreads) combine_lone_kernel(const __grid_constant__ CombineArgs args) {
-  const CombineOp& op = args.op[blockIdx.y];
-  const RankCtx& c = *op.ctx;
-  const int H = c.hidden, K = c.topk;
+struct LoneCombineArgs {
+  CombineOp op;
+  RankCtx ctx;
+  char* heap;
+  SlotLayout layout;
+};
+
+__global__ void __launch_bounds__(kLoneThreads) combine_lone_kernel(const __grid_constant__ LoneCombineArgs args) {
+  const CombineOp& op = args.op;
+  const RankCtx& c = args.ctx;
+  const SlotLayout& sl = args.layout;
   const bool single_round = c.single_round != 0;
   const int tid = threadIdx.x, lane = tid & 31;
-  char* const my_heap = c.heap[c.rank];
-  CtrlHeader* const hdr = header_of(my_heap);
-  const SlotLayout sl = slot_layout(op.slot_capacity, op.slot_tokens, H, K, 1);
-  char* const slot = my_heap + op.slot_off;
+  CtrlHeader* const hdr = header_of(args.heap);
+  char* const slot = args.heap + op.slot_off;
   const unsigned long long* const mask_arr = reinterpret_cast<const unsigned long long*>(slot + sl.mask);
   const int* const send_rows = reinterpret_cast<const int*>(slot + sl.send_rows);
   const int* const misc = reinterpret_cast<const int*>(slot + sl.misc);
   const char* const partial = reinterpret_cast<const char*>(op.partial);
   char* const out = reinterpret_cast<char*>(op.out);
-  const int fan = route_fanout(K, 1);
-  const long long row_bytes = static_cast<long long>(H) * 2;
+  const int row_vecs = c.hidden / 8;
+  const int units = (row_vecs + 32 * kLoneUnroll - 1) / (32 * kLoneUnroll);
+  wait_for_previous();
+  launch_dependents();
 
-  const unsigned e = ld_volatile_u32(&hdr->comb_epoch) + 1;
-  if (e > kLastEpoch) {
-    if (tid == 0 && blockIdx.x == 0) report_error(c, kEpochsExhausted, kPhaseCombine, 0xE0, e);
-    return;
+  unsigned e = 0, sample = ~0u;
+  int received = 0;
+  if (tid == 0) {
+    e = ld_volatile_u32(&hdr->comb_epoch) + 1;
+    received = misc[kValidCount];
+    if (op.samples != nullptr && e <= kLastEpoch) sample = sample_begin(op.samples, e, op.sample_capacity);
   }
-  const unsigned sample = sample_begin(op.samples, e, op.sample_capacity);
-  if (misc[kValidCount] > op.partial_rows && tid == 0 && blockIdx.x == 0)
-    report_error(c, kCapacityExceeded, kPhaseCombine, 7, static_cast<unsigned>(op.partial_rows));
-
-  const int warps = kLoneThreads / 32;
-  // Warp w of CTA c takes tokens w * grid + c, ...: every CTA (hence every SM) ends up with the
-  // same number of rows to within one, also when the grid was rounded up to whole waves.
-  for (long long t = static_cast<long long>(tid >> 5) * gridDim.x + blockIdx.x; t < op.tokens;
-       t += static_cast<long long>(gridDim.x) * warps) {
-    const int row = (mask_arr[t] & 1ull) ? send_rows[t * fan] : -1;
+  // Fan-out one: token t's record is mask_arr[t] and send_rows[t]. Unit i of the batch goes to warp
+  // i % warps, so every CTA (hence every SM) gets the same number of units to within one.
+  const unsigned warps = gridDim.x * (kLoneThreads / 32);
+  const unsigned long long items = static_cast<unsigned long long>(op.tokens) * units;
+  for (unsigned long long item = static_cast<unsigned>(tid >> 5) * gridDim.x + blockIdx.x; item < items; item += warps) {
+    const unsigned t = static_cast<unsigned>(item / units);
+    const int first = static_cast<int>(item - static_cast<unsigned long long>(t) * units) * 32 * kLoneUnroll + lane;
+    const int at = send_rows[t];                                  // independent of the mask: both loads are in flight
+    const int row = (mask_arr[t] & 1ull) ? at : -1;
     const bool usable = row >= 0 && row < op.partial_rows;       // warp-uniform
-    const char* src = partial + static_cast<long long>(usable ? row : 0) * row_bytes;
-    char* dst = out + t * row_bytes;
-    for (long long base = static_cast<long long>(lane) * 16; base < row_bytes; base += 32ll * 16 * kLoneUnroll) {
-      Chunk<4> v[kLoneUnroll] = {};
+    const char* src = partial + static_cast<long long>(usable ? row : 0) * row_vecs * 16;
+    char* dst = out + static_cast<long long>(t) * row_vecs * 16;
+    Chunk<4> v[kLoneUnroll] = {};
 #pragma unroll
-      for (int u = 0; u < kLoneUnroll; ++u) {
-        const long long off = base + static_cast<long long>(u) * 512;
-        if (usable && off < row_bytes) v[u] = load_local_chunk<4>(src + off);
-      }
+    for (int u = 0; u < kLoneUnroll; ++u)
+      if (usable && first + u * 32 < row_vecs) v[u] = load_local_chunk<4>(src + (first + u * 32) * 16ll);
 #pragma unroll
-      for (int u = 0; u < kLoneUnroll; ++u) {
-        const long long off = base + static_cast<long long>(u) * 512;
-        if (off >= row_bytes) continue;
-        unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
-        Chunk<4> result;
-        if (!usable) {
-          result = finish<4>(acc, v[u], false, single_round);          // no contributor: zeros
-        } else if (single_round) {
-          accumulate<4>(acc, v[u]);
-          result = finish<4>(acc, v[u], false, true);
-        } else {
-          result = finish<4>(acc, v[u], true, false);
-        }
-        store_chunk<4>(dst + off, result);
+    for (int u = 0; u < kLoneUnroll; ++u) {
+      if (first + u * 32 >= row_vecs) continue;
+      unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+      Chunk<4> result;
+      if (!usable) {
+        result = finish<4>(acc, v[u], false, single_round);          // no contributor: zeros
+      } else if (single_round) {
+        accumulate<4>(acc, v[u]);
+        result = finish<4>(acc, v[u], false, true);
+      } else {
+        result = finish<4>(acc, v[u], true, false);
       }
+      store_chunk<4>(dst + (first + u * 32) * 16ll, result);
     }
   }
-
-  __syncthreads();
-  sample_end(op.samples, sample);
+  // The epoch moves on once every CTA has read it. (Its load was in flight while the rows moved.)
+  if (op.samples != nullptr) __syncthreads();
   if (tid == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(&hdr->cfin_count, 1u);
-    if (prev == gridDim.x - 1) {
-      hdr->cdone_count = 0;
+    if (e > kLastEpoch) {
+      if (blockIdx.x == 0) report_error(c, kEpochsExhausted, kPhaseCombine, 0xE0, e);
+      return;
+    }
+    if (blockIdx.x == 0 && received > op.partial_rows)
+      report_error(c, kCapacityExceeded, kPhaseCombine, 7, static_cast<unsigned>(op.partial_rows));
+    sample_end(op.samples, sample);
+    if (atomicAdd(&hdr->cfin_count, 1u) == gridDim.x - 1) {
       hdr->cfin_count = 0;
-      hdr->cwork_push = 0;
-      hdr->cwork_reduce = 0;
       hdr->comb_epoch = e;
-      __threadfence();
     }
   }
 }
@@ -1184,20 +1190,21 @@ bool combine_can_mailbox(bool vec16, int fanout, int world, long long row_bytes)
   return vec16 && fanout <= kPeerBatch && world > 1 && row_bytes <= static_cast<long long>(kPushStages) * kPushStageBytes;
 }
 
-cudaError_t launch_combine(const CombineArgs& args, int ranks, int ctas_per_rank, bool vec16, int fanout, int world,
-                           int hidden, bool mailbox, bool cooperative, cudaStream_t stream) {
+cudaError_t launch_combine(const CombineArgs& args, int ranks, int ctas_per_rank, bool vec16, int fanout,
+                           const RankCtx& host_ctx, bool mailbox, bool cooperative, cudaStream_t stream) {
+  const int world = host_ctx.world;
   void* params[] = {const_cast<CombineArgs*>(&args)};
   CombineVariant variant;
-  const long long row_bytes = static_cast<long long>(hidden) * 2;
+  const long long row_bytes = static_cast<long long>(host_ctx.hidden) * 2;
   if (world == 1 && ranks == 1 && vec16 && args.op[0].profile == nullptr) {
-    // One rank: a streaming pass over local memory, one token per warp and pass.
-    const int warps = kLoneThreads / 32, tokens = args.op[0].tokens;
-    int ctas = (tokens + warps - 1) / warps;
-    if (ctas < 1) ctas = 1;
+    // One rank: a streaming pass over local memory in 2 KB units.
+    const long long warps = kLoneThreads / 32, unit = 32 * kLoneUnroll * 16;
+    const long long wanted = (args.op[0].tokens * ((row_bytes + unit - 1) / unit) + warps - 1) / warps;
+    int ctas = wanted < 1 ? 1 : (wanted > kLoneMaxCtas ? kLoneMaxCtas : static_cast<int>(wanted));
     if (ctas > kLoneSms) ctas = (ctas + kLoneSms - 1) / kLoneSms * kLoneSms;   // whole waves over the SMs
-    if (ctas > kLoneMaxCtas) ctas = kLoneMaxCtas;
-    return cudaLaunchKernel(reinterpret_cast<const void*>(combine_lone_kernel), dim3(ctas, 1, 1),
-                            dim3(kLoneThreads, 1, 1), params, 0, stream);
+    LoneCombineArgs lone_args{args.op[0], host_ctx, host_ctx.heap[host_ctx.rank], {}};
+    lone_args.layout = slot_layout(args.op[0].slot_capacity, args.op[0].slot_tokens, host_ctx.hidden, host_ctx.topk, 1);
+    return launch_chained(combine_lone_kernel, ctas, kLoneThreads, 1, 0, stream, lone_args);
   }
   cudaError_t err = pick_combine(vec16, fanout, mailbox && combine_can_mailbox(vec16, fanout, world, row_bytes), &variant,
                                  args.op[0].profile != nullptr);

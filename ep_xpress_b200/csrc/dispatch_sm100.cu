@@ -673,6 +673,289 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_kernel(const __grid_cons
   dispatch_body<IdT, kVec16, kProfile>(args.op[blockIdx.y], tile_base);
 }
 
+// ---- a group of ONE rank ----------------------------------------------------------------------
+// The destination of every live token is the rank's own receive plane, so dispatch is a compaction
+// copy and what the general kernel spends before its first row moves - routes of 512-token tiles on
+// a few CTAs, a rank-wide barrier, the tile prefix, claims from a counter - is most of its distance
+// from the copy bound. Here CTA c owns tokens [T c / ctas, T (c + 1) / ctas): it routes them, its
+// movers start to load, and it publishes how many of them are live as one tagged word and sums the
+// words of all CTAs (one round trip, hidden under the loads). A batch of at most 512 tokens is routed by every CTA and needs no exchange.
+// The payload is bound by HBM (or L2): eight movers with a ring of three 7 KB pieces each keep 172 KB
+// per SM in flight, and a stage is refilled as soon as its own store has read it.
+constexpr int kLoneMovers = 8;
+constexpr int kLoneStages = 3;
+constexpr int kLonePieceBytes = 7168;
+constexpr size_t kLoneSmemBytes = static_cast<size_t>(kLoneMovers) * kLoneStages * kLonePieceBytes;
+constexpr int kMetaThreads = kThreads - 32 * kLoneMovers;
+constexpr int kLoneMaxCtas = 512;
+constexpr unsigned kLoneTag = 0x80000000u;   // no generation and no row position has this bit
+
+struct LoneDispatchArgs {
+  DispatchOp op;
+  RankCtx ctx;
+  char* heap;
+  SlotLayout layout;
+};
+
+// All but the `kLeft` youngest bulk-copy groups of this thread have read their source.
+template <int kLeft>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kLeft) : "memory"); }
+
+// Whether a token of a group of one rank has a row; invalid ids or weights raise `bad`.
+template <typename IdT>
+__device__ __forceinline__ bool lone_route(const DispatchOp& op, int K, int E, int t, bool* bad) {
+  const long long row = static_cast<long long>(t) * K;
+  bool live = false, wrong = false;
+  if (K <= kRegK) {
+    long long id[kRegK];
+    float w[kRegK];
+#pragma unroll
+    for (int k = 0; k < kRegK; ++k) {
+      id[k] = k < K ? load_id<IdT>(op.ids, row + k) : -1;
+      w[k] = k < K ? op.weights[row + k] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < kRegK; ++k) {
+      const bool in_range = id[k] >= 0 && id[k] < E;
+      if (id[k] != -1 && (!in_range || !isfinite(w[k]))) wrong = true;
+      live |= in_range;
+#pragma unroll
+      for (int j = 0; j < k; ++j)
+        if (id[k] >= 0 && id[j] == id[k]) wrong = true;
+    }
+  } else {
+    for (int k = 0; k < K; ++k) {
+      const long long id = load_id<IdT>(op.ids, row + k);
+      if (id == -1) continue;
+      if (id < 0 || id >= E) { wrong = true; continue; }
+      if (!isfinite(op.weights[row + k])) wrong = true;
+      for (int j = 0; j < k; ++j)
+        if (load_id<IdT>(op.ids, row + j) == id) wrong = true;
+      live = true;
+    }
+  }
+  *bad = wrong;
+  return live && !wrong;
+}
+
+template <typename IdT>
+__global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid_constant__ LoneDispatchArgs args) {
+  extern __shared__ __align__(128) char lone_smem[];
+  const DispatchOp& op = args.op;
+  const RankCtx& c = args.ctx;            // by value: a context or a layout behind a pointer is a dependent load more
+  const SlotLayout& sl = args.layout;
+  const int H = c.hidden, K = c.topk, E = c.num_experts;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int T = op.tokens, ctas = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
+  char* const my_heap = args.heap;
+  CtrlHeader* const hdr = header_of(my_heap);
+  char* const slot = my_heap + op.slot_off;
+  int* const misc = reinterpret_cast<int*>(slot + sl.misc);
+  const long long row_bytes = static_cast<long long>(H) * 2;
+  const int first = static_cast<int>(static_cast<long long>(T) * cta / ctas);
+  const int mine = static_cast<int>(static_cast<long long>(T) * (cta + 1) / ctas) - first;   // <= kThreads
+
+  __shared__ int s_row[kThreads];         // receive row of each of this CTA's tokens, -1: none
+  __shared__ int s_warp_cnt[kWarps];
+  __shared__ int s_base, s_total, s_dirty;
+  __shared__ unsigned long long s_full[kLoneMovers * kLoneStages];
+
+  launch_dependents();
+  const unsigned g = ld_volatile_u32(&hdr->disp_epoch) + 1;
+
+  // ---- movers: warp w takes pieces w, w + kLoneMovers, ... of the CTA's rows ----------------
+  const int pieces = static_cast<int>((row_bytes + kLonePieceBytes - 1) / kLonePieceBytes);
+  const int piece_bytes = static_cast<int>(align_up((row_bytes + pieces - 1) / pieces, 16));
+  const int items = mine * pieces;
+  const bool mover = warp < kLoneMovers;
+  char* const ring = lone_smem + static_cast<size_t>(mover ? warp : 0) * kLoneStages * kLonePieceBytes;
+  unsigned long long* const full = s_full + (mover ? warp : 0) * kLoneStages;
+  unsigned loading = 0, parity = 0;       // bit s: a load into stage s is in flight; phase of its barrier
+  auto load_piece = [&](int item, int stage) {
+    const int token = item / pieces;
+    const long long b0 = static_cast<long long>(item - token * pieces) * piece_bytes;
+    const unsigned bytes = static_cast<unsigned>(min(row_bytes, b0 + piece_bytes) - b0);
+    mbarrier_arrive_expect_tx(full + stage, bytes);
+    bulk_load_to_smem(ring + static_cast<size_t>(stage) * kLonePieceBytes,
+                      reinterpret_cast<const char*>(op.x) + (first + token) * row_bytes + b0, bytes, full + stage);
+    loading |= 1u << stage;
+  };
+
+  // ---- route ---------------------------------------------------------------------------------------
+  if (tid == kThreads - 1) {
+    s_base = 0;
+    s_total = 0;
+    s_dirty = misc[kDirtyRows];
+  }
+  bool ok = g <= kLastEpoch;              // uniform over the launch; nothing is received after the last generation
+  if (!ok && tid == 0 && cta == 0) report_error(c, kEpochsExhausted, kPhaseDispatch, 0xE0, g);
+  const unsigned sample = ok ? sample_begin(op.samples, g, op.sample_capacity) : ~0u;
+  const bool solo = T <= kThreads;
+  const int t = solo ? tid : first + tid;
+  const bool routed = solo ? tid < T : tid < mine;
+  bool bad = false;
+  const bool live = routed && lone_route<IdT>(op, K, E, t, &bad);
+  if (bad) report_error(c, kInvalidRoute, kPhaseDispatch, 1, static_cast<unsigned>(t));
+  const unsigned ballot = __ballot_sync(0xffffffffu, live);
+  if (lane == 0) s_warp_cnt[warp] = __popc(ballot);
+  __syncthreads();
+  int at = __popc(ballot & ((1u << lane) - 1u)), counted = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    const int v = s_warp_cnt[w];
+    if (w < warp) at += v;
+    counted += v;
+  }
+  // The first loads leave once the routes are in: issued before them, they made the ids wait for 25 MB
+  // of payload (4096 x 7168: routed after 5.5 us instead of 2.3). They are in flight while the counts
+  // are exchanged.
+  if (mover && lane == 0 && ok) {         // the mover's lane 0 alone touches its barriers and its ring
+    for (int s = 0; s < kLoneStages; ++s) mbarrier_init(full + s, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+    for (int s = 0; s < kLoneStages; ++s)
+      if (warp + s * kLoneMovers < items) load_piece(warp + s * kLoneMovers, s);
+  }
+  int base = 0, total = counted;
+  const int me = tid - 32 * kLoneMovers;  // index among the threads that do not move payload
+  if (!solo && ok) {
+    // Words of other generations carry another tag, and the general kernel's positions, which share
+    // the plane, never have the tag's top bit.
+    unsigned long long* const words = reinterpret_cast<unsigned long long*>(slot + sl.dest_rows);
+    if (me == 0) st_release_gpu_u64(words + cta, tagged(g | kLoneTag, static_cast<unsigned>(counted)));
+    // Polled with plain volatile loads, a warp's words in one request: an acquire per word of every
+    // CTA queues 22,000 requests at ten cache lines. Only the values are used.
+    int before = 0, all = 0;
+    for (int i = me; i >= 0 && i < ctas && ok; i += kMetaThreads) {
+      unsigned long long word = 0;
+      ok = bounded_wait(c, kPhaseDispatch, 3, [&] {
+        word = ld_volatile_u64(words + i);
+        return tag_of(word) == (g | kLoneTag);
+      });
+      all += static_cast<int>(value_of(word));
+      if (i < cta) before += static_cast<int>(value_of(word));
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    all = __reduce_add_sync(0xffffffffu, all);
+    if (lane == 0 && !mover) {
+      atomicAdd(&s_base, before);
+      atomicAdd(&s_total, all);
+    }
+    ok = __syncthreads_and(ok);
+    base = s_base;
+    total = s_total;
+  }
+  const bool fits = total <= op.capacity && op.capacity <= op.slot_capacity;
+  const int valid = fits ? total : 0;
+  const int dirty_prev = s_dirty;
+  if (ok && cta == 0 && tid == kThreads - 33) {
+    reinterpret_cast<unsigned long long*>(slot + sl.peer_off)[0] = op.slot_off;
+    reinterpret_cast<int*>(slot + sl.peer_cap)[0] = op.slot_capacity;
+    reinterpret_cast<int*>(slot + sl.send_cnt)[0] = valid;
+    reinterpret_cast<int*>(slot + sl.recv_cnt)[0] = total;
+    if (!fits) report_error(c, kCapacityExceeded, kPhaseDispatch, 0, static_cast<unsigned>(total));
+  }
+  if (routed && t >= first && t < first + mine) {
+    const int row = live && fits && ok ? base + at : -1;
+    s_row[t - first] = row;
+    reinterpret_cast<unsigned long long*>(slot + sl.mask)[t] = live ? 1ull : 0ull;
+    reinterpret_cast<int*>(slot + sl.send_rows)[t] = row;
+  }
+  __syncthreads();
+  debug_delay(c, 2);
+
+  // ---- payload ---------------------------------------------------------------------------------------
+  if (mover) {
+    if (lane == 0) {
+      int stage = 0;
+      for (int item = warp; item < items; item += kLoneMovers) {
+        const int token = item / pieces;
+        if ((loading >> stage) & 1u) {
+          if (!mbarrier_wait_bounded(full + stage, (parity >> stage) & 1u, c.timeout_ns)) {
+            report_error(c, kTimeout, kPhaseDispatch, 8, static_cast<unsigned>(first + token));
+            break;
+          }
+          loading &= ~(1u << stage);
+          parity ^= 1u << stage;
+          const int row = s_row[token];
+          if (row >= 0) {
+            // (The piece never meets the generic proxy: loaded and stored by the copy engine.)
+            const long long b0 = static_cast<long long>(item - token * pieces) * piece_bytes;
+            bulk_store_from_smem(slot + sl.hidden + row * row_bytes + b0, ring + static_cast<size_t>(stage) * kLonePieceBytes,
+                                 static_cast<unsigned>(min(row_bytes, b0 + piece_bytes) - b0));
+          }
+        }
+        bulk_commit_group();
+        // The stage before this one is free once every store but the one just issued has read its source.
+        const int previous = stage == 0 ? kLoneStages - 1 : stage - 1;
+        const int refill = item + (kLoneStages - 1) * kLoneMovers;
+        if (item != warp && refill < items && s_row[refill / pieces] >= 0) {
+          bulk_wait_read<1>();
+          load_piece(refill, previous);
+        }
+        if (++stage == kLoneStages) stage = 0;
+      }
+      bulk_wait_all_complete();
+    }
+  } else {
+    if (ok && tid == kThreads - 1) {
+      // The epoch and the dirty count may change once every CTA has read them: with the count words of
+      // all CTAs in, or, for a batch without an exchange, in the CTA that arrives here last. (Nobody
+      // waits for these words inside the launch, so they need not wait for the payload.)
+      bool closes = cta == 0;
+      if (solo) {
+        __threadfence();
+        closes = atomicAdd(&hdr->done_count, 1u) == static_cast<unsigned>(ctas) - 1u;
+        __threadfence();
+      } else {
+        __threadfence();
+      }
+      if (closes) {
+        misc[kValidCount] = valid;
+        misc[kDirtyRows] = valid;
+        hdr->done_count = 0;
+        hdr->disp_epoch = g;
+      }
+    }
+    // Row metadata, one (token, slot) per thread; then the padding rows of the slot's previous use.
+    long long* const ids_out = reinterpret_cast<long long*>(slot + sl.ids);
+    float* const w_out = reinterpret_cast<float*>(slot + sl.weights);
+    long long* const inv_out = reinterpret_cast<long long*>(slot + sl.inverse);
+    for (int i = me; i < mine * K; i += kMetaThreads) {
+      const int token = i / K, k = i - token * K;
+      const long long row = s_row[token];
+      if (row < 0) continue;
+      const long long source = static_cast<long long>(first + token) * K + k;
+      const long long id = load_id<IdT>(op.ids, source);
+      ids_out[row * K + k] = id >= 0 ? c.expert_local[id] : -1;
+      w_out[row * K + k] = id >= 0 ? op.weights[source] : 0.f;
+      if (k == 0) {
+        inv_out[row * 2] = c.rank;
+        inv_out[row * 2 + 1] = first + token;
+        reinterpret_cast<int*>(slot + sl.ret)[row] = first + token;
+      }
+    }
+    if (dirty_prev > valid && ok) {
+      const long long pad_rows = dirty_prev - valid;
+      const long long threads = static_cast<long long>(ctas) * kMetaThreads;
+      const long long from = static_cast<long long>(cta) * kMetaThreads + me;
+      for (long long i = from; i < pad_rows * K; i += threads) {
+        ids_out[static_cast<long long>(valid) * K + i] = -1;
+        w_out[static_cast<long long>(valid) * K + i] = 0.f;
+      }
+      for (long long i = from; i < pad_rows * 2; i += threads) inv_out[static_cast<long long>(valid) * 2 + i] = -1;
+      if (op.zero_padding) {
+        char* const pad = slot + sl.hidden + valid * row_bytes;
+        const long long vecs = pad_rows * row_bytes / 16;
+        for (long long i = from; i < vecs; i += threads) st_payload16(pad + i * 16, make_uint4(0, 0, 0, 0));
+      }
+    }
+  }
+  debug_delay(c, 3);
+  if (op.samples != nullptr) __syncthreads();   // the operation ends with its last mover
+  sample_end(op.samples, sample);
+}
+
 using DispatchKernel = void (*)(const DispatchArgs);
 
 // The profiling specialisations are separate kernels: an ordinary launch carries no timers.
@@ -712,8 +995,32 @@ cudaError_t dispatch_max_ctas(bool ids64, bool vec16, size_t dynamic_smem, int* 
   return cudaSuccess;
 }
 
-cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, int ctas_per_rank, bool ids64, bool vec16,
-                            size_t dynamic_smem, bool cooperative, cudaStream_t stream) {
+// A group of one rank takes its own kernel, except where that kernel's plan does not hold: rows that
+// are not 16-byte aligned (bulk copies), profiled operations (phase stamps of the general kernel),
+// more than 512 tokens per CTA (one thread routes one), and slots too small for the count words.
+static bool lone_applies(const DispatchArgs& args, int ranks, int world, int ctas, bool vec16) {
+  const DispatchOp& op = args.op[0];
+  if (world != 1 || ranks != 1 || !vec16 || op.profile != nullptr || ctas > kLoneMaxCtas) return false;
+  if (op.tokens <= kThreads) return true;
+  return op.tokens <= static_cast<long long>(ctas) * kThreads && 2 * ctas <= op.slot_tokens;
+}
+
+cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, const RankCtx& host_ctx, int ctas_per_rank, bool ids64,
+                            bool vec16, size_t dynamic_smem, bool cooperative, cudaStream_t stream) {
+  if (lone_applies(args, ranks, host_ctx.world, ctas_per_rank, vec16)) {
+    LoneDispatchArgs lone_args{args.op[0], host_ctx, host_ctx.heap[host_ctx.rank], {}};
+    lone_args.layout = slot_layout(args.op[0].slot_capacity, args.op[0].slot_tokens, host_ctx.hidden, host_ctx.topk, 1);
+    const auto lone = ids64 ? dispatch_lone_kernel<long long> : dispatch_lone_kernel<int>;
+    cudaError_t err = cudaFuncSetAttribute(lone, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLoneSmemBytes));
+    if (err != cudaSuccess) return err;
+    void* lone_params[] = {&lone_args};
+    // A batch that every CTA routes itself has no CTA waiting for another: a plain launch is enough.
+    if (!cooperative || args.op[0].tokens <= kThreads)
+      return cudaLaunchKernel(reinterpret_cast<const void*>(lone), dim3(ctas_per_rank, 1, 1), dim3(kThreads, 1, 1),
+                              lone_params, kLoneSmemBytes, stream);
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lone), dim3(ctas_per_rank, 1, 1),
+                                       dim3(kThreads, 1, 1), lone_params, kLoneSmemBytes, stream);
+  }
   DispatchKernel kernel = pick_kernel(ids64, vec16, args.op[0].profile != nullptr);
   if (dynamic_smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -235,7 +235,7 @@ class Engine {
     attach_samples(samples, n, [&](size_t i, unsigned long long* ring, int capacity) {
       args.op[i].samples = ring; args.op[i].sample_capacity = capacity;
     });
-    cuda_check(launch_dispatch(args, static_cast<int>(n), ctas, ids64, vec16, smem, cooperative_, stream_of(stream)),
+    cuda_check(launch_dispatch(args, static_cast<int>(n), host_ctx_[0], ctas, ids64, vec16, smem, cooperative_, stream_of(stream)),
                "dispatch launch");
   }
 
@@ -298,7 +298,7 @@ class Engine {
       args.op[i].samples = ring; args.op[i].sample_capacity = capacity;
     });
     const int fanout = route_fanout(topk_, world_);
-    cuda_check(launch_combine(args, static_cast<int>(n), ctas, vec16, fanout, world_, hidden_, mailbox < 0 ? streaming_ != 0 : mailbox != 0, cooperative_,
+    cuda_check(launch_combine(args, static_cast<int>(n), ctas, vec16, fanout, host_ctx_[0], mailbox < 0 ? streaming_ != 0 : mailbox != 0, cooperative_,
                               stream_of(stream)), "combine launch");
   }
 

@@ -48,6 +48,9 @@ __device__ __forceinline__ unsigned long long ld_acquire_gpu_u64(const unsigned 
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void st_release_gpu_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ int ld_volatile_i32(const int* p) {
   int v;
   asm volatile("ld.volatile.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -56,6 +59,11 @@ __device__ __forceinline__ int ld_volatile_i32(const int* p) {
 __device__ __forceinline__ unsigned ld_volatile_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.volatile.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ unsigned long long global_timer_ns() {
@@ -320,6 +328,33 @@ __device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, un
 }
 __device__ __forceinline__ unsigned long long bf16x2_to_f32x2(unsigned pair) {
   return pack_f32x2(__uint_as_float(pair << 16), __uint_as_float(pair & 0xffff0000u));
+}
+
+// Programmatic dependent launch: the next kernel of the chain may start its prologue / everything
+// the previous kernel wrote is visible from here on. (Both return at once in an ordinary launch.)
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Programmatic dependent launch: the kernel's dispatch and prologue overlap the tail of the kernel
+// before it on the stream. Kernels launched this way call wait_for_previous before they touch data,
+// and launch_dependents only after that, so a kernel that runs knows every earlier one is complete.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(Params...), int ctas, int threads, int cluster, size_t smem,
+                           cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(ctas, 1, 1);
+  config.blockDim = dim3(threads, 1, 1);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2]{};
+  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[0].val.programmaticStreamSerializationAllowed = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = cluster;
+  attributes[1].val.clusterDim.y = 1;
+  attributes[1].val.clusterDim.z = 1;
+  config.attrs = attributes;
+  config.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
 }  // namespace epx

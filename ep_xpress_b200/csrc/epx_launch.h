@@ -22,16 +22,17 @@ cudaError_t combine_max_ctas(bool vec16, int fanout, int* ctas);
 // resident together) over a plain launch (cheaper to enqueue; co-residency then rests on the
 // grid fitting the device, which the caller bounds with the *_max_ctas queries, and on no
 // other kernel holding the SMs forever).
-cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, int ctas_per_rank, bool ids64, bool vec16,
-                            size_t dynamic_smem, bool cooperative, cudaStream_t stream);
+// `host_ctx`: host copy of the first rank's context.
+cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, const RankCtx& host_ctx, int ctas_per_rank, bool ids64,
+                            bool vec16, size_t dynamic_smem, bool cooperative, cudaStream_t stream);
 // `mailbox`: push and reduce run side by side in every CTA (pusher warps move rows with bulk
 // copies and release one arrival word per row; the other warps reduce a token as soon as the
 // rows it is owed are in) instead of one after the other. It applies to 16-byte rows, fan-outs
 // up to eight, rows of up to 112 KiB and groups of two or more ranks (`combine_can_mailbox`); elsewhere, and when not
 // asked for, the sequential protocol runs. All ranks of a group must choose the same protocol.
 bool combine_can_mailbox(bool vec16, int fanout, int world, long long row_bytes);
-cudaError_t launch_combine(const CombineArgs& args, int ranks, int ctas_per_rank, bool vec16, int fanout, int world,
-                           int hidden, bool mailbox, bool cooperative, cudaStream_t stream);
+cudaError_t launch_combine(const CombineArgs& args, int ranks, int ctas_per_rank, bool vec16, int fanout,
+                           const RankCtx& host_ctx, bool mailbox, bool cooperative, cudaStream_t stream);
 
 // Synthetic expert used by the validation harness and the communication
 // benchmark: partial[row] = bf16(hidden[row] * sum_k weights[row,k] * factor[local_ids[row,k]])

@@ -152,10 +152,6 @@ __device__ __forceinline__ void umma_commit_pair(unsigned long long* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(smem_address(bar)), "h"(static_cast<unsigned short>(3)) : "memory");
 }
-// Programmatic dependent launch: the next kernel of the chain may start its prologue / everything
-// the previous kernel wrote is visible from here on. (Both return at once in an ordinary launch.)
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- the grouped GEMM kernel -------------------------------------------------------------------
 struct GemmParams {
@@ -650,28 +646,6 @@ bool make_gate_up_map(CUtensorMap* map, const void* base, int experts, int inter
   return encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box,
                         element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// A launch of the runner's chain: programmatic dependent launch, so that the kernel's prologue
-// overlaps the tail of the one before it (every kernel of the chain waits before it touches data).
-template <typename... Params, typename... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), int ctas, int threads, int cluster, size_t smem,
-                           cudaStream_t stream, Args... args) {
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(ctas, 1, 1);
-  config.blockDim = dim3(threads, 1, 1);
-  config.dynamicSmemBytes = smem;
-  config.stream = stream;
-  cudaLaunchAttribute attributes[2]{};
-  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attributes[0].val.programmaticStreamSerializationAllowed = 1;
-  attributes[1].id = cudaLaunchAttributeClusterDimension;
-  attributes[1].val.clusterDim.x = cluster;
-  attributes[1].val.clusterDim.y = 1;
-  attributes[1].val.clusterDim.z = 1;
-  config.attrs = attributes;
-  config.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
 }
 
 // Ring geometry: small batches use narrow token boxes and more stages.

@@ -143,6 +143,23 @@ def test_one_rank_group_streams_local_rows(hidden, tokens, rounding):
             assert group.status()[0][0] != 0
 
 
+@pytest.mark.parametrize("tokens,hidden,topk,ctas", [
+    (1, 64, 2, 1), (512, 264, 8, 3), (513, 264, 8, 3), (600, 3592, 3, 2), (1021, 3584, 9, 148), (700, 258, 4, 7),
+])
+def test_one_rank_dispatch_at_the_edges_of_its_plan(tokens, hidden, topk, ctas):
+    """Batches routed by every CTA (up to 512 tokens) and by shares, one and several pieces per row,
+    rows the bulk copies cannot take, tokens without a route, a smaller batch after a larger one."""
+    cfg = Config(hidden_size=hidden, topk=topk, max_tokens_per_rank=tokens, timeout_seconds=2.0)
+    emap = workloads.round_robin_expert_map(16, 1)
+    with EmulatedGroup(1, emap, cfg) as group:
+        slot = group.create_slot()
+        for seed, n in enumerate((tokens, max(1, tokens - 37), 0, tokens)):
+            ids, weights = workloads.uniform_routing(n, 16, topk, seed=seed, rank=0)
+            ids[torch.rand(n, generator=torch.Generator().manual_seed(seed)) < 0.2 * seed] = -1
+            xs = [workloads.gaussian_payload(n, hidden, seed=seed, rank=0)]
+            run_round(group, slot, xs, [ids if seed % 2 else ids.to(torch.int32)], [weights], emap, ctas=ctas)
+
+
 def test_intermediate_rounding_is_observable():
     """remote-sum -> bf16 -> + local -> bf16 differs from a single rounding on chosen values."""
     world, hidden = 3, 64
