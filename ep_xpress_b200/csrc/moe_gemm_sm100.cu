@@ -230,8 +230,14 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
   tcgen05_fence_after();
   const unsigned tmem_base = tmem_base_slot;
 
-  wait_for_previous();
-  launch_dependents();
+  // The tile list comes from the align step, which is complete before the launch right behind it lets
+  // this kernel start; only the tokens (and, when gathered, the list itself) are the previous kernel's.
+  // So the producer fills its ring with the first tile's WEIGHTS while the previous kernel ends, and
+  // waits before the first token load. Every thread waits before it leaves.
+  if (p.gather_rows != nullptr || warp != 0) {
+    wait_for_previous();
+    launch_dependents();
+  }
   const int total = p.counters[0] * p.m_tiles;
   const int pair_id = blockIdx.x / 2, pairs = gridDim.x / 2;
 
@@ -276,6 +282,17 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         }
       }
     } else if (elect_one()) {
+      int ahead = 0;                                 // k-steps of the first tile whose weights are under way
+      if (pair_id < total) {
+        const int tt = pair_id / p.m_tiles, mt = pair_id - tt * p.m_tiles;
+        const int4 tile = p.tiles[tt];
+        const unsigned tx = 2u * (kABytes + (8u << box_index(((tile.z + 15) & ~15) / 2)) * kTileK * 2);
+        for (; ahead < stages && ahead < p.k_steps; ++ahead) {
+          if (rank == 0) mbarrier_arrive_expect_tx(full_bar + ahead, tx);
+          load_weights(smem + static_cast<size_t>(ahead) * stage_bytes, ahead, tile.x, mt, peer_smem_address(full_bar + ahead, 0));
+        }
+      }
+      wait_for_previous();
       for (int item = pair_id; item < total && !failed; item += pairs) {
         const int tt = item / p.m_tiles, mt = item - tt * p.m_tiles;
         const int4 tile = p.tiles[tt];
@@ -287,9 +304,13 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
         for (int k = 0; k < p.k_steps; ++k) {
           unsigned char* a_dst = smem + static_cast<size_t>(s) * stage_bytes;
           const unsigned leader_full = peer_smem_address(full_bar + s, 0);
-          if (!mbar_wait(empty_bar + s, parity)) { failed = 1; break; }
-          if (rank == 0) mbarrier_arrive_expect_tx(full_bar + s, tx);
-          load_weights(a_dst, k, tile.x, mt, leader_full);
+          if (ahead > 0) {
+            --ahead;
+          } else {
+            if (!mbar_wait(empty_bar + s, parity)) { failed = 1; break; }
+            if (rank == 0) mbarrier_arrive_expect_tx(full_bar + s, tx);
+            load_weights(a_dst, k, tile.x, mt, leader_full);
+          }
           tma_load_2d_pair(a_dst + kABytes, map_b, k * kTileK, b_row, leader_full);
           if (++s == stages) { s = 0; parity ^= 1u; }
         }
@@ -538,61 +559,60 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const uint4* __restric
   }
 }
 
-// partial[row] = the row's local slots of y added in slot order; two slots' loads are in flight at a
-// time. A unit per warp instead of a row per warp: one decode row of eight slots 51 -> 5 us, 128 rows
-// 68 -> 7 us (one warp walked 56 dependent loads); large batches are HBM bound either way (4096 rows
-// x 8 slots, 529 MB: about 110 us).
+// partial[row] = the row's local slots of y added in slot order. A warp takes kVecs vectors per lane of
+// a row and keeps kSlots slots' loads in flight. Large batches are HBM bound with <4, 2> (2 KB units;
+// 4096 rows x 8 slots, 529 MB: about 110 us); a decode batch is a chain of latencies, and <1, 8> makes
+// the eight slots of a row one round trip instead of four and spreads it over four times the warps.
+template <int kVecs, int kSlots>
 __global__ void __launch_bounds__(256) moe_slot_sum_kernel(const uint4* __restrict__ y, const int* __restrict__ entry_pos,
                                                            const int* __restrict__ valid_count, uint4* __restrict__ partial,
                                                            int rows, int topk, int vecs_per_row) {
   wait_for_previous();
   launch_dependents();
   const int lane = threadIdx.x & 31;
-  const unsigned units = units_per_row(vecs_per_row);
+  const unsigned units = (vecs_per_row + 32 * kVecs - 1) / (32 * kVecs);
   const unsigned items = min(*valid_count, rows) * units;
   const unsigned warps = gridDim.x * (blockDim.x / 32);
   for (unsigned item = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); item < items; item += warps) {
     const unsigned row = item / units;
-    const int base = static_cast<int>(item - row * units) * kUnitVecs + lane;
+    const int base = static_cast<int>(item - row * units) * 32 * kVecs + lane;
     const int* positions = entry_pos + static_cast<long long>(row) * topk;
-    unsigned long long acc[4][4];
+    unsigned long long acc[kVecs][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < kVecs; ++u)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[u][i] = 0ull;
-    auto fetch = [&](uint4 (&v)[4], int pos) {
-      const uint4* src = y + static_cast<long long>(pos) * vecs_per_row;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (base + u * 32 < vecs_per_row) v[u] = src[base + u * 32];
-    };
-    auto add = [&](const uint4 (&v)[4]) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        acc[u][0] = add_f32x2(acc[u][0], bf16x2_to_f32x2(v[u].x));
-        acc[u][1] = add_f32x2(acc[u][1], bf16x2_to_f32x2(v[u].y));
-        acc[u][2] = add_f32x2(acc[u][2], bf16x2_to_f32x2(v[u].z));
-        acc[u][3] = add_f32x2(acc[u][3], bf16x2_to_f32x2(v[u].w));
-      }
-    };
     for (int k0 = 0; k0 < topk; k0 += 32) {
       const int mine = k0 + lane < topk ? positions[k0 + lane] : -1;
       unsigned local = __ballot_sync(0xffffffffu, mine >= 0);
       while (local != 0) {
-        uint4 first[4] = {}, second[4] = {};
-        fetch(first, __shfl_sync(0xffffffffu, mine, __ffs(local) - 1));
-        local &= local - 1;
-        const bool two = local != 0;
-        if (two) {
-          fetch(second, __shfl_sync(0xffffffffu, mine, __ffs(local) - 1));
+        uint4 v[kSlots][kVecs] = {};
+        unsigned taken = 0;
+#pragma unroll
+        for (int j = 0; j < kSlots; ++j) {
+          if (local == 0) break;                       // warp-uniform
+          const uint4* src = y + static_cast<long long>(__shfl_sync(0xffffffffu, mine, __ffs(local) - 1)) * vecs_per_row;
           local &= local - 1;
+          taken |= 1u << j;
+#pragma unroll
+          for (int u = 0; u < kVecs; ++u)
+            if (base + u * 32 < vecs_per_row) v[j][u] = src[base + u * 32];
         }
-        add(first);
-        if (two) add(second);
+#pragma unroll
+        for (int j = 0; j < kSlots; ++j) {
+          if (!((taken >> j) & 1u)) break;
+#pragma unroll
+          for (int u = 0; u < kVecs; ++u) {
+            acc[u][0] = add_f32x2(acc[u][0], bf16x2_to_f32x2(v[j][u].x));
+            acc[u][1] = add_f32x2(acc[u][1], bf16x2_to_f32x2(v[j][u].y));
+            acc[u][2] = add_f32x2(acc[u][2], bf16x2_to_f32x2(v[j][u].z));
+            acc[u][3] = add_f32x2(acc[u][3], bf16x2_to_f32x2(v[j][u].w));
+          }
+        }
       }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < kVecs; ++u) {
       if (base + u * 32 >= vecs_per_row) continue;
       unsigned out[4];
 #pragma unroll
@@ -769,9 +789,14 @@ cudaError_t launch_moe_slot_sum(const void* y, const int* entry_pos, const int* 
                                 int rows, int topk, int hidden_size, cudaStream_t stream) {
   if (hidden_size % 8) return cudaErrorInvalidValue;
   if (rows <= 0) return cudaSuccess;
-  return launch_chained(moe_slot_sum_kernel, mover_ctas(rows, hidden_size), 256, 1, 0, stream,
-                        static_cast<const uint4*>(y), entry_pos, valid_count, static_cast<uint4*>(partial), rows, topk,
-                        hidden_size / 8);
+  // One wave of warps with one vector per lane, or the streaming form.
+  const int vecs = hidden_size / 8;
+  const long long small = static_cast<long long>(rows) * ((vecs + 31) / 32);
+  if (small <= 148 * 64)
+    return launch_chained(moe_slot_sum_kernel<1, 8>, static_cast<int>((small + 7) / 8), 256, 1, 0, stream,
+                          static_cast<const uint4*>(y), entry_pos, valid_count, static_cast<uint4*>(partial), rows, topk, vecs);
+  return launch_chained(moe_slot_sum_kernel<4, 2>, mover_ctas(rows, hidden_size), 256, 1, 0, stream,
+                        static_cast<const uint4*>(y), entry_pos, valid_count, static_cast<uint4*>(partial), rows, topk, vecs);
 }
 
 }  // namespace epx
