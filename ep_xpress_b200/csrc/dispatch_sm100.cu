@@ -685,6 +685,7 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_kernel(const __grid_cons
 constexpr int kLoneMovers = 8;
 constexpr int kLoneStages = 3;
 constexpr int kLonePieceBytes = 7168;
+constexpr int kEarlyStages = 1;
 constexpr size_t kLoneSmemBytes = static_cast<size_t>(kLoneMovers) * kLoneStages * kLonePieceBytes;
 constexpr int kMetaThreads = kThreads - 32 * kLoneMovers;
 constexpr int kLoneMaxCtas = 512;
@@ -806,14 +807,13 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
     if (w < warp) at += v;
     counted += v;
   }
-  // The first loads leave once the routes are in: issued before them, they made the ids wait for 25 MB
-  // of payload (4096 x 7168: routed after 5.5 us instead of 2.3). They are in flight while the counts
-  // are exchanged.
+  // The ids were loaded before any payload, and the counts are exchanged with only kEarlyStages of the
+  // ring in flight: words of a few bytes queue behind payload on their way to memory.
   if (mover && lane == 0 && ok) {         // the mover's lane 0 alone touches its barriers and its ring
     for (int s = 0; s < kLoneStages; ++s) mbarrier_init(full + s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
-    for (int s = 0; s < kLoneStages; ++s)
+    for (int s = 0; s < kEarlyStages; ++s)
       if (warp + s * kLoneMovers < items) load_piece(warp + s * kLoneMovers, s);
   }
   int base = 0, total = counted;
@@ -867,6 +867,10 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
   // ---- payload ---------------------------------------------------------------------------------------
   if (mover) {
     if (lane == 0) {
+      for (int s = kEarlyStages; s < kLoneStages; ++s) {
+        const int item = warp + s * kLoneMovers;
+        if (item < items && s_row[item / pieces] >= 0) load_piece(item, s);
+      }
       int stage = 0;
       for (int item = warp; item < items; item += kLoneMovers) {
         const int token = item / pieces;

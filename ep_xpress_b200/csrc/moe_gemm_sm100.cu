@@ -736,6 +736,7 @@ cudaError_t launch_moe_gemm_gate_up(const void* sorted_x, const void* w13, void*
                                     int experts, int hidden_size, int inter_size, int sms, cudaStream_t stream,
                                     const int* gather_rows, long long gather_height) {
   if (hidden_size % kTileK || inter_size % kMoeGateUpTile) return cudaErrorInvalidValue;
+  if (rows <= 0) return cudaSuccess;     // (no scatter launch stands between this kernel and the align step then)
   if (gather_rows != nullptr && (gather_height <= 0 || gather_height >= (1ll << 31))) return cudaErrorInvalidValue;
   if (encode_tiled() == nullptr) return cudaErrorNotSupported;
   GemmMaps maps{};
@@ -766,6 +767,7 @@ cudaError_t launch_moe_gemm_down(const void* act, const void* w2, void* y, const
                                  long long max_sorted_rows, int experts, int hidden_size, int inter_size, int sms,
                                  cudaStream_t stream) {
   if (inter_size % kTileK || hidden_size % kMoeDownTile) return cudaErrorInvalidValue;
+  if (rows <= 0) return cudaSuccess;
   if (encode_tiled() == nullptr) return cudaErrorNotSupported;
   GemmMaps maps{};
   GemmParams params{};
