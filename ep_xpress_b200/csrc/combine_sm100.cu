@@ -21,17 +21,15 @@
 // launches (host_sm.cu:559-590, :1212-1468, :592-607) and, like its mailbox kernel
 // (host_sm.cu:1952-2511), receives and reduces in the same kernel. Default protocol
 // ("mailbox", groups of two or more ranks, 16-byte rows, fan-out up to eight):
-//   push     some CTAs of the launch only push: their pusher warp claims received rows whose
-//            token lives on a peer, fifteen per round. A row travels partial -> shared
-//            memory -> the owner's staging row as bulk asynchronous copies (TMA, no tensor
-//            map); when the copies of a round have completed, the pusher stores the
-//            combine epoch into the arrival word that sits right behind each staging row
-//            (one system-scope fence per round). No CTA-wide fence, no counter, no "all
-//            rows are out" message.
-//   reduce   at the same time the other CTAs walk the rank's own tokens:
-//            a producer warp polls the arrival words of exactly the rows a token is
-//            owed (local memory), copies them into a shared-memory stage, and four
-//            consumer warps add them in rank order and store the result.
+//   push     some CTAs of the launch only push received rows whose token lives on a peer, and store
+//            the combine epoch into the arrival word right behind each staging row once the row is
+//            complete there. Large batches: one warp claims fifteen rows per round, which travel
+//            partial -> shared memory -> staging row as bulk asynchronous copies (TMA, no tensor
+//            map); a round completes and is published while the next one loads. Small batches: all
+//            warps move rows through registers. No counter, no "all rows are out" message.
+//   reduce   at the same time the warps of the other CTAs walk the rank's own tokens: they poll
+//            the arrival words of exactly the rows a token is owed (local memory), add the rows
+//            in rank order and store the result.
 // The sequential protocol (push everything, fence, one progress word per peer, wait,
 // reduce) is kept for rows that are not 16-byte aligned, wider fan-outs, and as a
 // selectable fallback. A group of one rank only reduces.
@@ -213,13 +211,10 @@ constexpr int kMaxGroupStages = 3;
 constexpr int kChunksPerThread = 4;
 constexpr int kSegMaxBytes = 16384;               // largest row segment of one item
 
-// Mailbox protocol: the CTAs of a launch split into PUSH CTAs and REDUCE CTAs. A push CTA runs
-// one pusher warp that owns the whole shared memory as fifteen row stages; a reduce CTA runs
-// four reduce pipelines. The roles live on different SMs because they disturb each other on one:
-// every bulk copy of an SM goes through that SM's one copy engine, where the reducers' loads
-// queue behind peer stores that the saturated link drains slowly (measured: 3.8 us per reduce
-// item next to a pusher, 1.1 us alone), and the system-scope fence in front of a round's
-// arrival words waits for every store the SM has in flight.
+// Mailbox protocol: the CTAs of a launch split into PUSH CTAs and REDUCE CTAs. A push CTA of a large
+// batch runs one pusher warp that owns the whole shared memory as fifteen row stages; in a small batch
+// and in a reduce CTA every warp works on its own. The roles live on different SMs because the
+// system-scope fence in front of arrival words waits for every store its SM has in flight.
 //
 // That fence is the price of a release at system scope: it does not complete while its SM has
 // peer stores in flight and holds up the SM's next stores meanwhile (measured at 2 GPUs, 4096
@@ -228,15 +223,16 @@ constexpr int kSegMaxBytes = 16384;               // largest row segment of one 
 // few CTAs of the launch hold one herald warp per pusher - which runs the fence and stores the
 // arrival words while the pusher already moves its next round. (A herald warp inside the push
 // CTA or inside a reduce CTA does not help: the fence stalls whichever SM runs it, and a busy
-// SM's fence is as slow as the pusher's own.) Small batches, one round per pusher, keep the
-// fence in the pusher: the hand-over would only add latency.
-constexpr int kMailGroups = kMaxGroups;
+// SM's fence is as slow as the pusher's own.) Small batches keep the fence in the push CTA: the
+// hand-over would only add latency.
+//
+// Ranks emulated on one GPU, us of the kernel, with the reduce as stage rings, one fence per row or
+// herald warp and rounds one after the other -> now: 4 x 128 x 7168 41 -> 26, 8 x 67 x 2048 (Zipf)
+// 47 -> 23, 4 x 1024 x 7168 154 -> 113.
 constexpr int kMailThreads = kBulkThreads;
-constexpr size_t kMailReduceSmem = kBulkSmemBytes;
 constexpr int kPushStages = 15;                   // bulk copies a pusher keeps in flight
 constexpr int kPushStageBytes = 14336;
-constexpr size_t kMailSmemBytes = static_cast<size_t>(kPushStages) * kPushStageBytes;   // >= kMailReduceSmem
-static_assert(kMailSmemBytes >= kMailReduceSmem, "a reduce CTA's rings must fit the launch's shared memory");
+constexpr size_t kMailSmemBytes = static_cast<size_t>(kPushStages) * kPushStageBytes;
 
 // Push CTAs of a mailbox launch of `ctas` CTAs (at least two): enough SMs to keep the link
 // busy - a pusher moves fifteen rows per round trip - and the rest reduce, which is the heavier
@@ -293,6 +289,8 @@ __device__ __forceinline__ void bulk_store_from_smem(void* dst, const void* src,
                "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Every bulk copy this thread committed has read its source (the stage may be refilled).
+__device__ __forceinline__ void bulk_wait_all_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 // Every bulk copy this thread committed has read its source AND its writes are complete.
 __device__ __forceinline__ void bulk_wait_all_complete() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
@@ -312,20 +310,14 @@ struct BulkReduceArgs {
   unsigned long long timeout_ns;
   unsigned long long* profile;
   int cta, ctas;          // this CTA's index among the CTAs that reduce, and their number
-  // mailbox launches only
-  const RankCtx* ctx;
-  unsigned epoch;
 };
 
 // Barriers and item slots are indexed [group][stage]. Returns false when a bounded wait gave up.
 // Called by the first kGroups * (kGroupWarps + kGroupProducers) warps of the CTA: consumers first,
 // then the producer warps, kGroupProducers per group. The producers of a group take its items
 // alternately (item k fills stage k % stages whoever issues it), because a producer's per-item
-// chain - arrival words, look-ups, barrier, copies - is longer than the consumers' arithmetic. kMailbox: the peers are still pushing while this runs, so before a
-// producer copies a token's rows, lane j waits (bounded) for the arrival word behind the staging
-// row of remote contributor j to carry this combine's epoch, and the CTAs take items round-robin
-// so that each of them owns tokens from every part of the batch.
-template <int kGroups, bool kMailbox, size_t kReduceSmem, bool kProfile>
+// chain - look-ups, barrier, copies - is longer than the consumers' arithmetic.
+template <int kGroups, size_t kReduceSmem, bool kProfile>
 __device__ __forceinline__ bool bulk_reduce(const BulkReduceArgs& a, char* smem, unsigned long long* full_all,
                                             unsigned long long* empty_all, StageItem* items_all,
                                             Profiler<kProfile>& prof) {
@@ -351,18 +343,15 @@ __device__ __forceinline__ bool bulk_reduce(const BulkReduceArgs& a, char* smem,
   unsigned long long* const full = full_all + group * kMaxGroupStages;
   unsigned long long* const empty = empty_all + group * kMaxGroupStages;
   StageItem* const slots = items_all + group * kMaxGroupStages;
-  // Items of this CTA are a contiguous range (local memory only: a static split is balanced),
-  // or every ctas-th item in mailbox launches; the groups take them round-robin.
-  const int lo = kMailbox ? a.cta : static_cast<int>(static_cast<long long>(items) * a.cta / a.ctas);
-  const int hi = static_cast<int>(static_cast<long long>(items) * (a.cta + 1) / a.ctas);
-  const int stride = kMailbox ? a.ctas : 1;
-  const int cta_items = kMailbox ? (items > lo ? (items - lo + stride - 1) / stride : 0)
-                                 : hi - static_cast<int>(static_cast<long long>(items) * a.cta / a.ctas);
+  // Items of this CTA are a contiguous range (local memory only: a static split is balanced); the
+  // groups take them round-robin.
+  const int lo = static_cast<int>(static_cast<long long>(items) * a.cta / a.ctas);
+  const int cta_items = static_cast<int>(static_cast<long long>(items) * (a.cta + 1) / a.ctas) - lo;
   const int mine = cta_items > group ? (cta_items - group + kGroups - 1) / kGroups : 0;
   long long waited = 0, worked = 0, stored = 0;   // profiling only: cycles spent waiting / working / in the store loop
   bool ok = true;
   if (producer) {
-    auto item_of = [&](int k) { return lo + (group + k * kGroups) * stride; };
+    auto item_of = [&](int k) { return lo + group + k * kGroups; };
     // Lane L loads the mask of item L of the batch, lane 8q + j the row of contributor j of
     // item 4r + q.
     auto load_batch = [&](int base, unsigned long long& mask, int (&rows)[8]) {
@@ -381,26 +370,11 @@ __device__ __forceinline__ bool bulk_reduce(const BulkReduceArgs& a, char* smem,
       if (base + 32 < mine) load_batch(base + 32, mask_next, rows_next);
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
-        // Mailbox: one look at the arrival words of the next four items (lane 8q + j: contributor
-        // j of item 4r + q), so that the words' latency is paid once per four items. A word that
-        // already carries the epoch is final; the others are polled again when their item is up.
-        unsigned early = a.epoch;
-        if (kMailbox) {
-          const unsigned long long mk = __shfl_sync(0xffffffffu, mask_now, 4 * r + (lane >> 3));
-          const int k = base + 4 * r + (lane >> 3), j = lane & 7;
-          if (k < mine && k % producers == turn && j < __popcll(mk) && rows_now[r] >= 0 &&
-              nth_set_bit(mk, j) != a.self) {
-            const long long tk = item_of(k) / rsegs;
-            early = ld_acquire_sys_u32(reinterpret_cast<const unsigned*>(a.staging + (tk * a.fan + j) * a.stride + a.row_bytes));
-          }
-          __syncwarp();        // the lane that copies a row is not the lane that looked at its word
-        }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int i = 4 * r + q;
           const unsigned long long m = __shfl_sync(0xffffffffu, mask_now, i);
           const int row = __shfl_sync(0xffffffffu, rows_now[r], q * 8 + (lane & 7));
-          const unsigned seen = __shfl_sync(0xffffffffu, early, q * 8 + (lane & 7));
           if (base + i >= mine || !ok) continue;                 // warp-uniform
           if ((base + i) % producers != turn) continue;          // the pipeline's other producer fills that stage
           use = static_cast<unsigned>(base + i);                 // stages are used in item order
@@ -429,25 +403,6 @@ __device__ __forceinline__ bool bulk_reduce(const BulkReduceArgs& a, char* smem,
             if (row >= 0 && !(is_self && row >= a.partial_rows))
               src = is_self ? a.partial + static_cast<long long>(row) * a.row_bytes
                             : a.staging + (static_cast<long long>(t) * a.fan + lane) * a.stride;
-          }
-          if (kMailbox) {
-            // Contributor `lane` is a peer: its row is in once the word behind it carries this epoch.
-            const bool remote = src != nullptr && !is_self;
-            bool fine = true;
-            const unsigned long long wait_begin = prof.on() && group == 0 && lane == 0 ? global_timer_ns() : 0ull;
-            if (remote && seen != a.epoch) {
-              const unsigned* word = reinterpret_cast<const unsigned*>(src + a.row_bytes);
-              if (ld_acquire_sys_u32(word) != a.epoch)
-                fine = bounded_wait(*a.ctx, kPhaseCombine, 5, [&] { return ld_acquire_sys_u32(word) == a.epoch; },
-                                    prof.poll_counter());
-            }
-            if (remote && fine) prof.first(kProfFirstReceive);
-            if (!__all_sync(0xffffffffu, fine)) {
-              ok = false;
-              continue;
-            }
-            if (wait_begin != 0ull) prof.count(kProfArrivalWait, global_timer_ns() - wait_begin);
-            fence_proxy_async();      // the rows were written by a peer; the copies below read them through the async proxy
           }
           const unsigned valid = __ballot_sync(0xffffffffu, src != nullptr);
           const unsigned self_vote = __ballot_sync(0xffffffffu, is_self);
@@ -617,13 +572,12 @@ __device__ __forceinline__ void push_item(const PushArgs& p, long long item, int
 // Run by the pusher warp of a push CTA; lane i < kPushStages owns stage i. Per round the
 // warp claims one piece per lane with a single atomic (a row of up to kPushStageBytes is one
 // piece; towards the end of the batch the rounds shrink to an even share of what is left),
-// every lane resolves its piece, loads it into its stage, stores it to the owner's
-// staging row and waits for its own copies to complete; then ONE system-scope fence orders the
-// round's completed rows before the arrival words, which the lanes that moved a row's last
-// piece store relaxed (a release per word would serialise a round trip to the peer per word).
+// every lane resolves its piece, loads it into its stage and stores it to the owner's
+// staging row. While the next round's claim, look-ups and loads are under way, the round's copies
+// complete and ONE system-scope fence orders its rows before the arrival words, which the lanes that
+// moved a row's last piece store relaxed (a release per word would serialise a round trip to the peer per word).
 // The copies run in the SM's copy engine; the lanes only issue and wait, in lockstep, so a
-// round costs one chain of latencies (claim, look-up, load, store + acknowledgement, fence)
-// whatever the number of rows in it.
+// round costs one chain of latencies (load, store) whatever the number of rows in it.
 __device__ __forceinline__ void st_release_gpu_u32(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -646,7 +600,46 @@ __device__ __forceinline__ bool mailbox_push(const PushArgs& p, const RankCtx& c
   unsigned parity = 0;                                  // of this lane's barrier
   unsigned round = 0;
   bool ok = true;
-  while (true) {
+  unsigned* pending = nullptr;         // this lane's arrival word of the round whose stores are under way
+  // Waits until that round's rows are complete at their owners and publishes their arrival words (or
+  // hands them to the herald). Returns false when a bounded wait gave up.
+  auto publish = [&]() -> bool {
+    bulk_wait_all_complete();
+    fence_proxy_async();               // the copies wrote through the async proxy; the words below are ordinary stores
+    unsigned* const word = pending;
+    pending = nullptr;
+    // A round that only met holes of the interleaved order completed no row: nothing to order,
+    // nothing to publish (all pieces of a row travel in one round).
+    if (!__any_sync(0xffffffffu, word != nullptr)) return true;
+    if (hand == nullptr) {
+      __threadfence_system();
+      if (word != nullptr) {
+        st_relaxed_sys_u32(word, epoch);
+        prof.first(kProfFirstPublish);
+      }
+      return true;
+    }
+    // The arrival words go to the herald warp, which publishes them behind a system-scope fence while
+    // this warp moves on. The pusher runs at most kPushSlotRounds rounds ahead of its herald.
+    if (lane == 0 && round >= kPushSlotRounds)
+      ok = bounded_wait(c, kPhaseCombine, 9, [&] {
+        return ld_acquire_gpu_u32(&hand->heralded) + kPushSlotRounds > round; }, prof.poll_counter());
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    if (lane < kPushRoundWords)
+      hand->words[round % kPushSlotRounds][lane] = reinterpret_cast<unsigned long long>(word);
+    __syncwarp();
+    if (lane == 0) st_release_gpu_u32(&hand->posted, round + 1);
+    ++round;
+    return true;
+  };
+  // Claims a round and resolves this lane's piece of it.
+  struct Piece {
+    const char* src;
+    char* dst;
+    unsigned* word;
+    int bytes;
+  };
+  auto resolve = [&](Piece* piece_of) -> bool {
     unsigned base = 0, take = per_round;
     if (lane == 0) {
       const long long left = items - static_cast<long long>(ld_volatile_u32(&hdr->cwork_push));
@@ -656,30 +649,45 @@ __device__ __forceinline__ bool mailbox_push(const PushArgs& p, const RankCtx& c
     }
     base = __shfl_sync(0xffffffffu, base, 0);
     take = __shfl_sync(0xffffffffu, take, 0);
-    if (static_cast<long long>(base) >= items) break;
+    *piece_of = Piece{nullptr, nullptr, nullptr, 0};
+    if (static_cast<long long>(base) >= items) return false;
     const long long item = static_cast<long long>(base) + lane;
-    char* dst = nullptr;
-    unsigned* word = nullptr;
-    int bytes = 0;
     if (lane < static_cast<int>(take) && item < items) {
       const int piece = static_cast<int>(item % pieces);
       long long row;
       int source;
       if (push_target(p, item / pieces, &row, &source)) {
         const long long b0 = static_cast<long long>(piece) * piece_bytes;
-        bytes = static_cast<int>(min(p.row_bytes, b0 + piece_bytes) - b0);
         char* dst_row = p.stage[source] + static_cast<long long>(p.ret[row]) * p.stride;
-        dst = dst_row + b0;
-        if (piece == pieces - 1) word = reinterpret_cast<unsigned*>(dst_row + p.row_bytes);
-        mbarrier_arrive_expect_tx(bar, static_cast<unsigned>(bytes));
-        bulk_load_to_smem(stage, p.partial + row * p.row_bytes + b0, static_cast<unsigned>(bytes), bar);
+        piece_of->src = p.partial + row * p.row_bytes + b0;
+        piece_of->dst = dst_row + b0;
+        piece_of->bytes = static_cast<int>(min(p.row_bytes, b0 + piece_bytes) - b0);
+        if (piece == pieces - 1) piece_of->word = reinterpret_cast<unsigned*>(dst_row + p.row_bytes);
       }
+    }
+    return true;
+  };
+  Piece now, next;
+  bool more = resolve(&now);
+  while (more) {
+    char* const dst = now.dst;
+    unsigned* const word = now.word;
+    const int bytes = now.bytes;
+    if (dst != nullptr) {
+      mbarrier_arrive_expect_tx(bar, static_cast<unsigned>(bytes));
+      bulk_load_to_smem(stage, now.src, static_cast<unsigned>(bytes), bar);
+    }
+    more = resolve(&next);             // the next round's claim and look-ups hide under this round's loads
+    now = next;
+    // The round before this one completes and is published while this round's loads are under way.
+    if (!publish()) {
+      if (dst != nullptr) mbarrier_wait_bounded(bar, parity, c.timeout_ns);   // this round's loads still target the stages
+      break;
     }
     const unsigned long long wait_begin = prof.on() && lane == 0 ? global_timer_ns() : 0ull;
     if (dst != nullptr) {
       if (mbarrier_wait_bounded(bar, parity, c.timeout_ns)) {
         parity ^= 1u;
-        fence_proxy_async();
         bulk_store_from_smem(dst, stage, static_cast<unsigned>(bytes));
         prof.moved(word != nullptr ? 1 : 0, static_cast<unsigned long long>(bytes));
       } else {
@@ -687,44 +695,25 @@ __device__ __forceinline__ bool mailbox_push(const PushArgs& p, const RankCtx& c
       }
     }
     bulk_commit_group();
-    bulk_wait_all_complete();
+    bulk_wait_all_read();              // the stage may be filled again
     if (wait_begin != 0ull) prof.count(kProfPushWait, global_timer_ns() - wait_begin);
-    fence_proxy_async();               // the copies wrote through the async proxy; the words below are ordinary stores
+    pending = word;
     if (!__all_sync(0xffffffffu, ok)) break;
-    // A round that only met holes of the interleaved order completed no row: nothing to order,
-    // nothing to publish (all pieces of a row travel in one round).
-    if (!__any_sync(0xffffffffu, word != nullptr)) continue;
-    if (hand == nullptr) {
-      __threadfence_system();
-      if (word != nullptr) {
-        st_relaxed_sys_u32(word, epoch);
-        prof.first(kProfFirstPublish);
-      }
-      continue;
-    }
-    // The round's rows are complete at their owners: its arrival words go to the herald warp,
-    // which publishes them behind a system-scope fence while this warp already moves the next
-    // round. The pusher runs at most kPushSlotRounds rounds ahead of its herald.
-    if (lane == 0 && round >= kPushSlotRounds)
-      ok = bounded_wait(c, kPhaseCombine, 9, [&] {
-        return ld_acquire_gpu_u32(&hand->heralded) + kPushSlotRounds > round; }, prof.poll_counter());
-    if (!__all_sync(0xffffffffu, ok)) break;
-    if (lane < kPushRoundWords)
-      hand->words[round % kPushSlotRounds][lane] = reinterpret_cast<unsigned long long>(word);
-    __syncwarp();
-    if (lane == 0) st_release_gpu_u32(&hand->posted, round + 1);
-    ++round;
   }
+  if (__all_sync(0xffffffffu, ok)) publish();
+  bulk_wait_all_complete();
   const bool fine = __all_sync(0xffffffffu, ok);
   if (hand != nullptr && lane == 0) st_release_gpu_u32(&hand->final_rounds, round + 1);
   return fine;
 }
 
-// The herald warp of ONE pusher, on an SM whose only stores are arrival words. Whenever the
-// pusher has posted rounds: ONE system-scope fence - cumulative over the pusher's completed
-// copies, which reached this warp through the release/acquire on `posted` - then the rounds'
-// arrival words as relaxed stores (lane l: the word of stage l). A release per word would
-// serialise a round trip to the peer per word.
+// The herald warps of a herald CTA, one per pusher, on an SM whose only stores are arrival words. Whenever
+// some pushers have posted rounds: ONE system-scope fence for the CTA - cumulative over those pushers'
+// completed copies, which reached its warps through the release/acquire on `posted` and then the
+// barrier - and every warp stores its pusher's arrival words relaxed (lane l: the word of stage l). A
+// release per word would serialise a round trip to the peer per word, and a fence per warp queues up
+// sixteen fences on the SM: the last words left 20 us after the last row. Called by all threads of the
+// CTA; `slot` is null in warps without a pusher.
 template <bool kProfile>
 __device__ __forceinline__ bool mailbox_herald(const RankCtx& c, PushSlot* slot, unsigned epoch, int lane,
                                                Profiler<kProfile>& prof) {
@@ -734,30 +723,185 @@ __device__ __forceinline__ bool mailbox_herald(const RankCtx& c, PushSlot* slot,
   while (true) {
     unsigned long long both = 0;
     // (posted, final_rounds) in one load; a pusher that is done posts nothing more.
-    if (lane == 0) both = ld_acquire_gpu_u64(reinterpret_cast<const unsigned long long*>(&slot->posted));
+    if (lane == 0 && slot != nullptr) both = ld_acquire_gpu_u64(reinterpret_cast<const unsigned long long*>(&slot->posted));
     both = __shfl_sync(0xffffffffu, both, 0);
     const unsigned posted = static_cast<unsigned>(both), final_rounds = static_cast<unsigned>(both >> 32);
-    if (posted == done) {
-      if (final_rounds != 0 && done + 1 == final_rounds) return true;
-      if ((++spins & 63u) == 0) {
-        if (ld_volatile_i32(&header_of(c.heap[c.rank])->abort_flag) != 0) return false;
-        if (global_timer_ns() - start > c.timeout_ns) return false;
+    if (__syncthreads_or(posted != done)) {
+      if (threadIdx.x == 0) __threadfence_system();
+      __syncthreads();
+      for (unsigned round = done; round != posted; ++round) {
+        unsigned long long word = 0;
+        if (lane < kPushRoundWords) word = ld_relaxed_sys(&slot->words[round % kPushSlotRounds][lane]);
+        if (word != 0ull) {
+          st_relaxed_sys_u32(reinterpret_cast<unsigned*>(word), epoch);
+          prof.first(kProfFirstPublish);
+        }
       }
+      __syncwarp();
+      if (lane == 0 && posted != done) st_release_gpu_u32(&slot->heralded, posted);
+      done = posted;
       continue;
     }
-    __threadfence_system();
-    for (unsigned round = done; round != posted; ++round) {
-      unsigned long long word = 0;
-      if (lane < kPushRoundWords) word = ld_relaxed_sys(&slot->words[round % kPushSlotRounds][lane]);
-      if (word != 0ull) {
-        st_relaxed_sys_u32(reinterpret_cast<unsigned*>(word), epoch);
-        prof.first(kProfFirstPublish);
+    if (__syncthreads_and(slot == nullptr || (final_rounds != 0 && done + 1 == final_rounds))) return true;
+    if ((++spins & 63u) == 0) {
+      const bool give_up = ld_volatile_i32(&header_of(c.heap[c.rank])->abort_flag) != 0 ||
+                           global_timer_ns() - start > c.timeout_ns;
+      if (__syncthreads_or(give_up)) return false;
+    }
+  }
+}
+
+// ---- mailbox push, small batches -------------------------------------------------------------
+// One round per pusher warp and nothing to overlap: what counts is the length of the chain. Every warp
+// of a push CTA moves whole rows through registers (look-up, loads, peer stores), one system-scope
+// fence orders two rows of every warp before their arrival words, so a CTA has 24 rows under way where the bulk-copy pusher has fifteen and a
+// copy through shared memory between each load and store; and it takes them from the received rows
+// themselves (the other ranks' rows, starting behind this rank's own), without holes and claims.
+template <bool kProfile>
+__device__ __forceinline__ void mailbox_push_rows(const PushArgs& p, unsigned epoch, int received, int warp, int warps,
+                                                  int lane, Profiler<kProfile>& prof) {
+  constexpr int kUnroll = 10;
+  constexpr int kRows = 2;             // rows of a warp per fence
+  const int own = p.rows_from[p.self], after_own = p.first_row[p.self] + own, count = received - own;
+  for (int begin = 0; begin < count; begin += kRows * warps) {        // the same trips for every warp
+    char* moved[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      moved[j] = nullptr;
+      const int i = begin + j * warps + warp;
+      int row = after_own + i;
+      if (row >= received) row -= received;
+      if (i >= count || row >= p.valid) continue;
+      const long long back = p.ret[row];
+      int source = 0;
+      for (int r = 1; r < p.world; ++r)
+        if (row >= p.first_row[r]) source = r;       // the last rank whose rows start at or before this one
+      const char* src = p.partial + row * p.row_bytes;
+      char* const dst = p.stage[source] + back * p.stride;
+      moved[j] = dst;
+      for (long long base = lane * 16; base < p.row_bytes; base += 32 * 16 * kUnroll) {
+        Chunk<4> v[kUnroll];
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u)
+          if (base + u * 512 < p.row_bytes) v[u] = load_local_chunk<4>(src + base + u * 512);
+#pragma unroll
+        for (int u = 0; u < kUnroll; ++u)
+          if (base + u * 512 < p.row_bytes) store_chunk<4>(dst + base + u * 512, v[u]);
       }
     }
-    __syncwarp();
-    done = posted;
-    if (lane == 0) st_release_gpu_u32(&slot->heralded, done);
+    // One fence for the CTA's rows, cumulative through the barrier: an SM runs its warps' system-scope
+    // fences one after the other.
+    __syncthreads();
+    if (threadIdx.x == 0) __threadfence_system();
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      if (moved[j] == nullptr || lane != 0) continue;
+      st_relaxed_sys_u32(reinterpret_cast<unsigned*>(moved[j] + p.row_bytes), epoch);
+      prof.first(kProfFirstPublish);
+      prof.moved(1, static_cast<unsigned long long>(p.row_bytes));
+    }
   }
+}
+
+// ---- mailbox reduce -----------------------------------------------------------------------------
+// Every warp of a reduce CTA is a reducer of its own: it takes (token, row segment) items, lane j waits
+// (bounded) for the arrival word behind the staging row of remote contributor j, and all lanes add the
+// rows from global memory with every contributor's loads in flight. 24 warps with eight 16-byte loads
+// per lane keep 98 KB per SM under way. (Stage rings filled by bulk copies, with producer and consumer
+// warps, moved a 14 KB item per 2.3 us and pipeline, 25 GB/s per SM: their barriers, look-ups and
+// four consumer warps were one serial chain per item.)
+// The look-ups of the next item are in flight while the current one is added. Items go round-robin over
+// the CTAs, so that each of them owns tokens from every part of the batch.
+template <int kPeers, int kUnroll>
+__device__ __forceinline__ void mailbox_add(const char* staged, long long stride, const char* local, unsigned valid,
+                                            int self_index, char* outp, long long b0, long long b1, int lane,
+                                            bool single_round) {
+  for (long long base = b0 + lane * 16; base < b1; base += 512 * kUnroll) {
+    // A contributor without a row reads as zeros, and adding +0 changes no FP32 sum that started at +0:
+    // every load is issued before the first add and nothing branches in between.
+    uint4 v[kPeers][kUnroll];
+#pragma unroll
+    for (int b = 0; b < kPeers; ++b) {
+      const char* const row = b == self_index ? local : staged + b * stride;
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        v[b][u] = make_uint4(0u, 0u, 0u, 0u);
+        if (((valid >> b) & 1u) && base + u * 512 < b1) v[b][u] = ld_payload16(row + base + u * 512);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      if (base + u * 512 >= b1) continue;
+      unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+      Chunk<4> own{};
+#pragma unroll
+      for (int b = 0; b < kPeers; ++b) {
+        Chunk<4> c{{v[b][u].x, v[b][u].y, v[b][u].z, v[b][u].w}};
+        if (b == self_index && !single_round) own = c;
+        else accumulate<4>(acc, c);
+      }
+      store_chunk<4>(outp + base + u * 512, finish<4>(acc, own, true, single_round));
+    }
+  }
+}
+
+template <bool kProfile>
+__device__ __forceinline__ bool mailbox_reduce(const BulkReduceArgs& a, const RankCtx& c, unsigned epoch, int warp,
+                                               int warps, int lane, Profiler<kProfile>& prof) {
+  // 2 KB segments, cut to what one round of loads covers (eight rows' worth of 512 bytes) while that
+  // leaves warps without an item.
+  int seg = 2048;
+  const int round = a.fan <= 2 ? 2048 : (a.fan <= 4 ? 1024 : 512);
+  const long long workers = static_cast<long long>(a.ctas) * warps;
+  while (seg > round && a.tokens * ((a.row_bytes + seg - 1) / seg) < 2 * workers) seg /= 2;
+  const int segs = static_cast<int>((a.row_bytes + seg - 1) / seg);
+  const long long items = static_cast<long long>(a.tokens) * segs;
+  long long item = static_cast<long long>(warp) * a.ctas + a.cta;
+  unsigned long long mask_next = 0;
+  int row_next = -1;
+  auto look_up = [&](long long i) {
+    const long long t = i / segs;
+    mask_next = i < items ? a.mask_arr[t] : 0ull;
+    row_next = i < items && lane < a.fan ? a.send_rows[t * a.fan + lane] : -1;
+  };
+  look_up(item);
+  for (; item < items; item += workers) {
+    const unsigned long long m = mask_next;
+    const int row = row_next;
+    look_up(item + workers);
+    const long long t = item / segs;
+    const long long b0 = (item - t * segs) * seg, b1 = min(a.row_bytes, b0 + seg);
+    const int n = __popcll(m);
+    const char* src = nullptr;
+    bool is_self = false, fine = true;
+    if (lane < n) {
+      is_self = nth_set_bit(m, lane) == a.self;
+      if (row >= 0 && !(is_self && row >= a.partial_rows))
+        src = is_self ? a.partial + static_cast<long long>(row) * a.row_bytes
+                      : a.staging + (t * a.fan + lane) * a.stride;
+      if (src != nullptr && !is_self) {
+        const unsigned long long wait_begin = prof.on() && warp == 0 ? global_timer_ns() : 0ull;
+        const unsigned* word = reinterpret_cast<const unsigned*>(src + a.row_bytes);
+        fine = bounded_wait(c, kPhaseCombine, 5, [&] { return ld_acquire_sys_u32(word) == epoch; }, prof.poll_counter());
+        if (fine) prof.first(kProfFirstReceive);
+        if (wait_begin != 0ull) prof.count(kProfArrivalWait, global_timer_ns() - wait_begin);
+      }
+    }
+    if (!__all_sync(0xffffffffu, fine)) return false;
+    if (lane == 0) prof.count(kProfItems, 1);
+    const unsigned valid = __ballot_sync(0xffffffffu, src != nullptr);
+    const unsigned vote = __ballot_sync(0xffffffffu, is_self);
+    const int self_index = vote != 0 ? __ffs(vote) - 1 : -1;
+    const unsigned long long local_bits = __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(src), self_index & 31);
+    const char* const local = reinterpret_cast<const char*>(local_bits);
+    const char* const staged = a.staging + t * a.fan * a.stride;
+    char* const outp = a.out + t * a.row_bytes;
+    if (n <= 2) mailbox_add<2, 4>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
+    else if (n <= 4) mailbox_add<4, 2>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
+    else mailbox_add<8, 1>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
+  }
+  return true;
 }
 
 enum CombineMode : int { kModeRegister = 0, kModeBulk = 1, kModeMailbox = 2 };
@@ -792,7 +936,7 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
   __shared__ char* s_stage[64];
   __shared__ int s_need[64];
   __shared__ int s_rows_from[64], s_first_row[64];
-  __shared__ int s_most;
+  __shared__ int s_most, s_received;
   __shared__ int s_last;
   __shared__ unsigned long long s_full[kMaxGroups * kMaxGroupStages], s_empty[kMaxGroups * kMaxGroupStages];
   __shared__ unsigned long long s_push_full[kPushStages + 1];
@@ -817,16 +961,32 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
     s_stage[tid] = c.heap[tid] + off + pl.staging;
     s_need[tid] = (tid != self && reinterpret_cast<const int*>(slot + sl.send_cnt)[tid] > 0) ? 1 : 0;
   }
-  if (tid == 64) {
-    int at = 0, most = 0;
-    for (int r = 0; r < W; ++r) {
-      const int count = reinterpret_cast<const int*>(slot + sl.recv_cnt)[r];
-      s_first_row[r] = at;
-      s_rows_from[r] = count;
-      at += count;
-      if (r != self && count > most) most = count;
+  if (tid >= 64 && tid < 96) {       // one warp: the counts in one round trip, two per lane
+    const int* const recv_cnt = reinterpret_cast<const int*>(slot + sl.recv_cnt);
+    const int low = lane < W ? recv_cnt[lane] : 0, high = lane + 32 < W ? recv_cnt[lane + 32] : 0;
+    int upto_low = low, upto_high = high;
+#pragma unroll
+    for (int step = 1; step < 32; step <<= 1) {
+      const int l = __shfl_up_sync(0xffffffffu, upto_low, step), h = __shfl_up_sync(0xffffffffu, upto_high, step);
+      if (lane >= step) {
+        upto_low += l;
+        upto_high += h;
+      }
     }
-    s_most = most;
+    const int all_low = __shfl_sync(0xffffffffu, upto_low, 31);
+    if (lane < W) {
+      s_first_row[lane] = upto_low - low;
+      s_rows_from[lane] = low;
+    }
+    if (lane + 32 < W) {
+      s_first_row[lane + 32] = all_low + upto_high - high;
+      s_rows_from[lane + 32] = high;
+    }
+    const int most = __reduce_max_sync(0xffffffffu, max(lane == self ? 0 : low, lane + 32 == self ? 0 : high));
+    if (lane == 31) {
+      s_most = most;
+      s_received = all_low + upto_high;
+    }
   }
   if (kBulk) {
     if (tid < kMaxGroups * kMaxGroupStages) {
@@ -856,9 +1016,6 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
   reduce.out = reinterpret_cast<char*>(op.out); reduce.row_bytes = row_bytes; reduce.stride = stride;
   reduce.tokens = T; reduce.fan = fan; reduce.self = self; reduce.partial_rows = op.partial_rows;
   reduce.single_round = single_round; reduce.timeout_ns = c.timeout_ns; reduce.profile = op.profile;
-  reduce.ctx = &c;
-  reduce.epoch = e;
-
   reduce.cta = static_cast<int>(blockIdx.x);
   reduce.ctas = static_cast<int>(gridDim.x);
   if (kMode == kModeMailbox) {
@@ -871,21 +1028,23 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
     const int cta = static_cast<int>(blockIdx.x);
     debug_delay(c, 4);
     if (cta < push_ctas) {
-      if (tid < 32) {
+      if (op.herald == 0) {
+        mailbox_push_rows<kProfile>(push, e, s_received, cta + (tid >> 5) * push_ctas, push_ctas * (kMailThreads / 32), lane, prof);
+      } else if (tid < 32) {
         if (!mailbox_push<kProfile>(push, c, hdr, dynamic_smem, s_push_full, e, heralds ? hand + cta : nullptr, lane,
                                     push_ctas, prof) && lane == 0)
           report_error(c, kTimeout, kPhaseCombine, 6, 0);
-        if (kProfile && prof.on() && lane == 0) prof.record[1] = global_timer_ns();
       }
+      if (kProfile && prof.on() && tid == 0) prof.record[1] = global_timer_ns();
     } else if (cta < push_ctas + herald_ctas) {
       const int pusher = (cta - push_ctas) * kHeraldWarpsPerCta + (tid >> 5);
-      if ((tid >> 5) < kHeraldWarpsPerCta && pusher < push_ctas &&
-          !mailbox_herald<kProfile>(c, hand + pusher, e, lane, prof) && lane == 0)
+      const bool owner = (tid >> 5) < kHeraldWarpsPerCta && pusher < push_ctas;
+      if (!mailbox_herald<kProfile>(c, owner ? hand + pusher : nullptr, e, lane, prof) && lane == 0)
         report_error(c, kTimeout, kPhaseCombine, 8, 0);
     } else {
       reduce.cta = cta - push_ctas - herald_ctas;
       reduce.ctas = static_cast<int>(gridDim.x) - push_ctas - herald_ctas;
-      if (!bulk_reduce<kMailGroups, true, kMailReduceSmem, kProfile>(reduce, dynamic_smem, s_full, s_empty, s_items, prof))
+      if (!mailbox_reduce<kProfile>(reduce, c, e, tid >> 5, kMailThreads / 32, lane, prof) && lane == 0)
         report_error(c, kTimeout, kPhaseCombine, 4, 0);
     }
   } else {
@@ -938,7 +1097,7 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
   // ---- D. rank-order reduce from local memory -----------------------------------------------
   if (kBulk) {
     fence_proxy_async();      // the rows were written by generic stores; the reduce reads them through the async proxy
-    if (!bulk_reduce<kMaxGroups, false, kBulkSmemBytes, kProfile>(reduce, dynamic_smem, s_full, s_empty, s_items, prof))
+    if (!bulk_reduce<kMaxGroups, kBulkSmemBytes, kProfile>(reduce, dynamic_smem, s_full, s_empty, s_items, prof))
       report_error(c, kTimeout, kPhaseCombine, 4, 0);
   } else {
     const long long items = static_cast<long long>(T) * segs;

@@ -364,10 +364,16 @@ __device__ __forceinline__ void dispatch_body(const DispatchOp& op, int* tile_ba
   if (tid < W) {
     const int d = tid;
     int off = 0, total = 0;
-    for (int s = 0; s < W && !lone; ++s) {
-      const int v = static_cast<int>(value_of(ld_relaxed_sys(my_cnt + s * W + d)));
-      if (s < self) off += v;
-      total += v;
+    for (int s0 = 0; s0 < W && !lone; s0 += 8) {        // eight words in flight at a time
+      unsigned long long word[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) word[i] = s0 + i < W ? ld_relaxed_sys(my_cnt + (s0 + i) * W + d) : 0ull;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int v = static_cast<int>(value_of(word[i]));
+        if (s0 + i < self) off += v;
+        total += v;
+      }
     }
     if (lone) total = s_send[0];
     const unsigned long long base = lone ? op.slot_off
