@@ -45,7 +45,8 @@ constexpr int kABytes = 128 * kTileK * 2;  // one CTA's weight rows of a k-step
 constexpr int kMaxStages = 12;
 constexpr int kRingBytes = 7 * (kABytes + kMaxTileN / 2 * kTileK * 2);   // 224 KB: seven stages of the widest tile
 constexpr size_t kGemmSmemBytes = kRingBytes + 1024;                      // + alignment of the swizzled tiles
-constexpr int kGemmThreads = 192;
+constexpr int kMaxEpilogueShare = 4;       // epilogue warps per TMEM lane quadrant
+constexpr int kGemmThreads = 64 + 128 * kMaxEpilogueShare;   // of the widest launch
 constexpr int kAccumColumns = 256;
 constexpr int kNMaps = 5;                  // boxes of 8, 16, 32, 64 and 128 token rows
 constexpr unsigned long long kGemmWaitNs = 2000000000ull;   // bound of every pipeline wait: 2 s
@@ -188,8 +189,12 @@ __device__ __forceinline__ int box_index(int half) {
 //
 // Persistent: pair c takes tiles c, c + pairs, ... in (token tile, weight tile) order, so the
 // pairs that run together share one expert's tokens and, for experts with several token tiles,
-// its weights in L2. Warp 0 feeds the ring, warp 1 issues MMAs, warps 2-5 drain the accumulators
-// (two buffers of 256 TMEM columns, so the epilogue of one tile overlaps the next main loop).
+// its weights in L2. Warp 0 feeds the ring, warp 1 issues MMAs, the others drain the accumulators
+// (two buffers of 256 TMEM columns, so the epilogue of one tile overlaps the next main loop): up to four
+// warps per TMEM lane quadrant, which take 32 tokens each in turn. The epilogue is about 500
+// instructions per 32 tokens; with one warp per quadrant it took 16,000 cycles for a wide tile, longer
+// than the main loop of K = 768 and as long as that of K = 2048, and stood alone at the end. (See
+// epilogue_shares for narrower tiles.)
 // Every wait is bounded and ends in an error flag, after which TMEM is still released.
 //
 // kMode 0: 256 weight rows = 128 gate and 128 up rows of the same columns, interleaved by 16, so
@@ -208,6 +213,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned rank = cluster_ctarank();           // 0 = leader
+  const int shares = (static_cast<int>(blockDim.x) - 64) / 128;
   const int stages = p.stages;
   const int stage_bytes = kABytes + p.b_rows * kTileK * 2;
   if (threadIdx.x == 0) {
@@ -217,7 +223,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
     }
     for (int b = 0; b < 2; ++b) {
       mbarrier_init(acc_full + b, 1);                // one commit from the leader per tile
-      mbarrier_init(acc_empty + b, 8);               // leader's: four epilogue warps of each CTA
+      mbarrier_init(acc_empty + b, 8 * shares);        // leader's: the epilogue warps of both CTAs
     }
     failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -347,7 +353,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
   } else {
     // ---------------- epilogue (both CTAs, own 128 weight rows) ----------------
     // TMEM lane = weight row (output column), TMEM column = token.
-    const int quadrant = warp & 3;
+    const int quadrant = warp & 3, share = (warp - 2) >> 2;
     unsigned local_tile = 0;
     for (int item = pair_id; item < total; item += pairs, ++local_tile) {
       const int tt = item / p.m_tiles, mt = item - tt * p.m_tiles;
@@ -362,7 +368,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
                                     : mt * kTileM + static_cast<int>(rank) * 128 + quadrant * 32 + lane;
       __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(tile.y) * p.out_columns + column;
 #pragma unroll 1
-      for (int c0 = 0; c0 < tile.z; c0 += 32) {
+      for (int c0 = 32 * share; c0 < tile.z; c0 += 32 * shares) {
         unsigned v[32];
         tmem_load_32(taddr + c0, v);
         tmem_load_wait();
@@ -675,12 +681,21 @@ void set_ring(GemmParams* params, int tile_cap) {
   params->stages = stages < kMaxStages ? stages : kMaxStages;
 }
 
+// Epilogue warps per quadrant: as many as tiles may need, each with 32 tokens. Narrow tiles are bound by
+// the weights' stream, and idle warps at the accumulator's barrier slow it down (hidden 7168, inter 2048,
+// 32 experts of 32 tokens: four warps 454 us a layer, two 446; 16 experts of 254 tokens, hidden 2048,
+// inter 768: one 88, two 83, four 78 us).
+int epilogue_shares(const GemmParams& params) {
+  const int cap = 2 * params.b_rows;
+  return cap >= kMaxTileN ? kMaxEpilogueShare : (cap >= 64 ? 2 : 1);
+}
+
 template <int kMode>
 cudaError_t launch_gemm(GemmMaps& maps, const GemmParams& params, int sms, cudaStream_t stream) {
   cudaError_t err = cudaFuncSetAttribute(grouped_gemm_kernel<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kGemmSmemBytes));
   if (err != cudaSuccess) return err;
-  return launch_chained(grouped_gemm_kernel<kMode>, sms / 2 * 2, kGemmThreads, 2, kGemmSmemBytes, stream, maps, params);
+  return launch_chained(grouped_gemm_kernel<kMode>, sms / 2 * 2, 64 + 128 * epilogue_shares(params), 2, kGemmSmemBytes, stream, maps, params);
 }
 
 }  // namespace
