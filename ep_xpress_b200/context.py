@@ -99,8 +99,9 @@ class Pending:
             raise ValueError("device tickets never block the host; timeout is not supported")
         self._check_workspace()
         context = self._context
-        with torch.cuda.device(context.device):
-            consumer = stream or torch.cuda.current_stream(context.device)
+        caller = getattr(context, "_caller_stream", None)
+        with context._on_device() if caller is not None else torch.cuda.device(context.device):
+            consumer = stream or (caller() if caller is not None else torch.cuda.current_stream(context.device))
             if consumer.device != context.device:
                 raise ValueError("completion stream must belong to the context device")
             consumer.wait_event(self._completed)

@@ -429,6 +429,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("THREADS") = kThreads;
   m.attr("PROFILE_STAMPS") = kProfileStamps;
   m.attr("SAMPLE_WORDS") = kSampleWords;
+  // BF16 [rows, columns] from the caching allocator's pool of `stream`, as torch.empty under that stream.
+  m.def("empty_rows", [](int64_t rows, int64_t columns, int device, int64_t stream) {
+    c10::cuda::CUDAStreamGuard guard(c10::cuda::getStreamFromExternal(stream_of(stream), static_cast<c10::DeviceIndex>(device)));
+    return at::empty({rows, columns}, at::TensorOptions().dtype(at::kBFloat16).device(at::kCUDA, device));
+  });
   m.def("heap_allocate", [](size_t bytes) { return reinterpret_cast<int64_t>(HeapRegistry::instance().allocate(bytes)); });
   m.def("heap_export", [](int64_t base) { return py::bytes(HeapRegistry::instance().export_handle(reinterpret_cast<void*>(base))); });
   m.def("heap_open", [](const std::string& handle, size_t bytes) {

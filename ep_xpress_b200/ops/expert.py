@@ -17,6 +17,8 @@ def scale_rows(context, batch, factors=None, out=None, stream=None):
     core = context._core
     if out is None:
         out = context.partial_buffer(batch.handle)
-    stream = stream or torch.cuda.current_stream(context.device)
+    if stream is None:
+        caller = getattr(context, "_caller_stream", None)
+        stream = caller() if caller is not None else torch.cuda.current_stream(context.device)
     core.scale_rows(batch.hidden, batch.local_ids, batch.weights, batch.valid_count, factors, out, stream)
     return out
