@@ -415,24 +415,27 @@ constexpr int kMaxLocalExperts = 1024;
 constexpr int kAlignClusterMax = 8;
 
 // Exclusive prefix sum over the CTA's 1024 threads (`warp_sums` is 32 words of shared memory).
-__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int upto = v;
+__device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
 #pragma unroll
   for (int step = 1; step < 32; step <<= 1) {
-    const int below = __shfl_up_sync(0xffffffffu, upto, step);
-    if (lane >= step) upto += below;
+    const int below = __shfl_up_sync(0xffffffffu, v, step);
+    if (lane >= step) v += below;
   }
+  return v;
+}
+__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int upto = warp_inclusive_scan(v, lane);
   __syncthreads();
   if (lane == 31) warp_sums[warp] = upto;
   __syncthreads();
-  int base = 0;
-  for (int w = 0; w < warp; ++w) base += warp_sums[w];
-  return base + upto - v;
+  const int sums = warp_inclusive_scan(warp_sums[lane], lane);      // every warp scans the 32 sums itself
+  const int below = __shfl_sync(0xffffffffu, sums, (warp + 31) & 31);
+  return (warp == 0 ? 0 : below) + upto - v;
 }
 
-// A chain of memory and barrier latencies, not bandwidth. One cluster of 1-8 CTAs packs the local (row, slot) pairs by expert: every CTA counts its share
-// of the pairs per expert in shared memory (the counting atomic also ranks the pair inside the
+// A chain of memory and barrier latencies, not bandwidth. One cluster of 1-8 CTAs packs the local
+// (row, slot) pairs by expert: every CTA counts its share of the pairs per expert in shared memory (the counting atomic also ranks the pair inside the
 // CTA), the CTAs read each other's counts through distributed shared memory, every CTA derives
 // the same prefix sums, and the second pass writes each pair to expert base + CTA base + rank.
 // Bounded by the device valid_count, never by a host-side count; order inside an expert is free
@@ -461,25 +464,45 @@ __global__ void __launch_bounds__(kAlignThreads) moe_align_kernel(const long lon
   const int pairs = min(*valid_count, rows) * topk;
   const int step = static_cast<int>(ctas) * kAlignThreads;
   constexpr int kBatch = 4;                          // independent loads in flight per thread
-  for (int first = static_cast<int>(cta) * kAlignThreads + tid; first < pairs; first += kBatch * step) {
+  // The first batch of a thread stays in registers between the two passes, weights included; up to
+  // 32768 pairs there is no other and the second pass loads nothing.
+  int held_id[kBatch], held_at[kBatch];
+  float held_weight[kBatch];
+  for (int first = static_cast<int>(cta) * kAlignThreads + tid, round = 0; first < pairs; first += kBatch * step, ++round) {
     long long id[kBatch];
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) id[b] = first + b * step < pairs ? local_ids[first + b * step] : -1;
+    if (round == 0) {
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) held_weight[b] = first + b * step < pairs ? weights[first + b * step] : 0.f;
+    }
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
-      if (first + b * step < pairs)
-        entry_pos[first + b * step] = id[b] >= 0 && id[b] < experts ? atomicAdd(&s_count[id[b]], 1) : -1;
+      const bool mine = id[b] >= 0 && id[b] < experts;
+      const int at = mine ? atomicAdd(&s_count[id[b]], 1) : -1;
+      if (round == 0) {
+        held_id[b] = mine ? static_cast<int>(id[b]) : 0;
+        held_at[b] = at;
+      } else if (first + b * step < pairs) {
+        entry_pos[first + b * step] = at;
+      }
     }
   }
   cluster_sync();
   // Thread e: rows of expert e in the whole cluster and in the CTAs before this one.
   int mine = 0, before = 0;
   if (tid < experts) {
-    for (unsigned c = 0; c < ctas; ++c) {
-      unsigned v;
-      asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_smem_address(s_count + tid, c)) : "memory");
-      mine += static_cast<int>(v);
-      if (c < cta) before += static_cast<int>(v);
+    unsigned v[kAlignClusterMax];
+#pragma unroll
+    for (unsigned c = 0; c < kAlignClusterMax; ++c) {  // all CTAs' counts in one round trip
+      v[c] = 0;
+      if (c < ctas)
+        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v[c]) : "r"(peer_smem_address(s_count + tid, c)) : "memory");
+    }
+#pragma unroll
+    for (unsigned c = 0; c < kAlignClusterMax; ++c) {
+      mine += static_cast<int>(v[c]);
+      if (c < cta) before += static_cast<int>(v[c]);
     }
   }
   const int offset = block_exclusive_scan(mine, s_scan);
@@ -499,21 +522,25 @@ __global__ void __launch_bounds__(kAlignThreads) moe_align_kernel(const long lon
     }
   }
   __syncthreads();
-  for (int first = static_cast<int>(cta) * kAlignThreads + tid; first < pairs; first += kBatch * step) {
-    int at[kBatch];
-    long long id[kBatch];
+  for (int first = static_cast<int>(cta) * kAlignThreads + tid, round = 0; first < pairs; first += kBatch * step, ++round) {
+    int at[kBatch], id[kBatch];
     float w[kBatch];
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
       const int i = first + b * step;
-      at[b] = i < pairs ? entry_pos[i] : -1;
-      id[b] = i < pairs ? local_ids[i] : -1;
-      w[b] = i < pairs ? weights[i] : 0.f;
+      const bool held = round == 0;
+      at[b] = held ? held_at[b] : (i < pairs ? entry_pos[i] : -1);
+      id[b] = held ? held_id[b] : (i < pairs ? static_cast<int>(local_ids[i]) : -1);
+      w[b] = held ? held_weight[b] : (i < pairs ? weights[i] : 0.f);
     }
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
       const int i = first + b * step;
-      if (at[b] < 0) continue;
+      if (i >= pairs) continue;
+      if (at[b] < 0) {
+        if (round == 0) entry_pos[i] = -1;
+        continue;
+      }
       const int pos = s_base[id[b]] + at[b];
       if (pos < max_sorted_rows) {
         sorted_row[pos] = i / topk;

@@ -44,6 +44,8 @@ def assert_elementwise_close(got, want):
     (1000, 8, 8, 1024, 384, 1000),
     (130, 8, 32, 256, 128, 0),
     (5, 2, 2, 256, 128, 3),
+    (300, 9, 16, 512, 128, 300),       # more slots than the slot sum keeps in flight
+    (10000, 4, 8, 256, 128, 9800),     # more pairs than the align step holds in registers, streaming slot sum
 ])
 def test_matches_fp32_reference(rows, topk, experts, hidden, inter, valid, gather_loads):
     x, ids, weights, count, w13, w2 = make_case(rows, topk, experts, hidden, inter, valid, seed=rows)
