@@ -685,7 +685,9 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_kernel(const __grid_cons
 // a few CTAs, a rank-wide barrier, the tile prefix, claims from a counter - is most of its distance
 // from the copy bound. Here CTA c owns tokens [T c / ctas, T (c + 1) / ctas): it routes them, its
 // movers start to load, and it publishes how many of them are live as one tagged word and sums the
-// words of all CTAs (one round trip, hidden under the loads). A batch of at most 512 tokens is routed by every CTA and needs no exchange.
+// words of all CTAs (one round trip, hidden under the loads). A batch of at most 768 tokens is routed by every CTA and needs no
+// exchange and no cooperative launch (hidden 2048, dispatch + expert + combine: 600 tokens 14.4 us, 17.3
+// with the exchange); every CTA routing 1024 costs more than that (18.5 us against 17.7).
 // The payload is bound by HBM (or L2): eight movers with a ring of three 7 KB pieces each keep 172 KB
 // per SM in flight, and a stage is refilled as soon as its own store has read it.
 constexpr int kLoneMovers = 8;
@@ -695,6 +697,7 @@ constexpr int kEarlyStages = 1;
 constexpr size_t kLoneSmemBytes = static_cast<size_t>(kLoneMovers) * kLoneStages * kLonePieceBytes;
 constexpr int kMetaThreads = kThreads - 32 * kLoneMovers;
 constexpr int kLoneMaxCtas = 512;
+constexpr int kSoloTokens = 768;          // batches that every CTA routes for itself
 constexpr unsigned kLoneTag = 0x80000000u;   // no generation and no row position has this bit
 
 struct LoneDispatchArgs {
@@ -763,8 +766,9 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
   const int mine = static_cast<int>(static_cast<long long>(T) * (cta + 1) / ctas) - first;   // <= kThreads
 
   __shared__ int s_row[kThreads];         // receive row of each of this CTA's tokens, -1: none
-  __shared__ int s_warp_cnt[kWarps];
-  __shared__ int s_base, s_total, s_dirty;
+  __shared__ unsigned s_live[kSoloTokens / 32];     // which of the routed tokens have a row
+  __shared__ int s_before[kSoloTokens / 32];        // ... and how many of them precede each word
+  __shared__ int s_base, s_total, s_dirty, s_counted;
   __shared__ unsigned long long s_full[kLoneMovers * kLoneStages];
 
   launch_dependents();
@@ -797,22 +801,31 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
   bool ok = g <= kLastEpoch;              // uniform over the launch; nothing is received after the last generation
   if (!ok && tid == 0 && cta == 0) report_error(c, kEpochsExhausted, kPhaseDispatch, 0xE0, g);
   const unsigned sample = ok ? sample_begin(op.samples, g, op.sample_capacity) : ~0u;
-  const bool solo = T <= kThreads;
-  const int t = solo ? tid : first + tid;
-  const bool routed = solo ? tid < T : tid < mine;
-  bool bad = false;
-  const bool live = routed && lone_route<IdT>(op, K, E, t, &bad);
-  if (bad) report_error(c, kInvalidRoute, kPhaseDispatch, 1, static_cast<unsigned>(t));
-  const unsigned ballot = __ballot_sync(0xffffffffu, live);
-  if (lane == 0) s_warp_cnt[warp] = __popc(ballot);
-  __syncthreads();
-  int at = __popc(ballot & ((1u << lane) - 1u)), counted = 0;
-#pragma unroll
-  for (int w = 0; w < kWarps; ++w) {
-    const int v = s_warp_cnt[w];
-    if (w < warp) at += v;
-    counted += v;
+  // Tokens this CTA routes: all of a small batch, else its own.
+  const bool solo = T <= kSoloTokens;
+  const int route_first = solo ? 0 : first, route_count = solo ? T : mine;
+  const int route_words = solo ? kSoloTokens / 32 : kWarps;
+  for (int i = tid; i < route_words * 32; i += kThreads) {
+    bool bad = false;
+    const bool live = i < route_count && lone_route<IdT>(op, K, E, route_first + i, &bad);
+    if (bad) report_error(c, kInvalidRoute, kPhaseDispatch, 1, static_cast<unsigned>(route_first + i));
+    const unsigned ballot = __ballot_sync(0xffffffffu, live);
+    if (lane == 0) s_live[i >> 5] = ballot;
   }
+  __syncthreads();
+  if (warp == kWarps - 1) {
+    const int v = lane < route_words ? __popc(s_live[lane]) : 0;
+    int upto = v;
+#pragma unroll
+    for (int step = 1; step < 32; step <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, upto, step);
+      if (lane >= step) upto += below;
+    }
+    if (lane < route_words) s_before[lane] = upto - v;
+    if (lane == 31) s_counted = upto;
+  }
+  __syncthreads();
+  const int counted = s_counted;
   // The ids were loaded before any payload, and the counts are exchanged with only kEarlyStages of the
   // ring in flight: words of a few bytes queue behind payload on their way to memory.
   if (mover && lane == 0 && ok) {         // the mover's lane 0 alone touches its barriers and its ring
@@ -861,9 +874,12 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
     reinterpret_cast<int*>(slot + sl.recv_cnt)[0] = total;
     if (!fits) report_error(c, kCapacityExceeded, kPhaseDispatch, 0, static_cast<unsigned>(total));
   }
-  if (routed && t >= first && t < first + mine) {
-    const int row = live && fits && ok ? base + at : -1;
-    s_row[t - first] = row;
+  if (tid < mine) {
+    const int t = first + tid, i = t - route_first;
+    const unsigned word = s_live[i >> 5], bit = 1u << (i & 31);
+    const bool live = (word & bit) != 0u;
+    const int row = live && fits && ok ? base + s_before[i >> 5] + __popc(word & (bit - 1u)) : -1;
+    s_row[tid] = row;
     reinterpret_cast<unsigned long long*>(slot + sl.mask)[t] = live ? 1ull : 0ull;
     reinterpret_cast<int*>(slot + sl.send_rows)[t] = row;
   }
@@ -1011,8 +1027,8 @@ cudaError_t dispatch_max_ctas(bool ids64, bool vec16, size_t dynamic_smem, int* 
 static bool lone_applies(const DispatchArgs& args, int ranks, int world, int ctas, bool vec16) {
   const DispatchOp& op = args.op[0];
   if (world != 1 || ranks != 1 || !vec16 || op.profile != nullptr || ctas > kLoneMaxCtas) return false;
-  if (op.tokens <= kThreads) return true;
-  return op.tokens <= static_cast<long long>(ctas) * kThreads && 2 * ctas <= op.slot_tokens;
+  if (op.tokens > static_cast<long long>(ctas) * kThreads) return false;
+  return op.tokens <= kSoloTokens || 2 * ctas <= op.slot_tokens;
 }
 
 cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, const RankCtx& host_ctx, int ctas_per_rank, bool ids64,
@@ -1025,7 +1041,7 @@ cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, const RankCtx& 
     if (err != cudaSuccess) return err;
     void* lone_params[] = {&lone_args};
     // A batch that every CTA routes itself has no CTA waiting for another: a plain launch is enough.
-    if (!cooperative || args.op[0].tokens <= kThreads)
+    if (!cooperative || args.op[0].tokens <= kSoloTokens)
       return cudaLaunchKernel(reinterpret_cast<const void*>(lone), dim3(ctas_per_rank, 1, 1), dim3(kThreads, 1, 1),
                               lone_params, kLoneSmemBytes, stream);
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lone), dim3(ctas_per_rank, 1, 1),
