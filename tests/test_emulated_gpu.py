@@ -161,6 +161,48 @@ def test_one_rank_dispatch_at_the_edges_of_its_plan(tokens, hidden, topk, ctas):
             run_round(group, slot, xs, [ids if seed % 2 else ids.to(torch.int32)], [weights], emap, ctas=ctas)
 
 
+def test_chained_launches_capture_behind_a_stream_fork():
+    """The kernels launched as programmatic dependents (expert, one-rank combine) as the first node of a
+    forked stream and as one with two predecessors: captured, replayed on new inputs, bit-exact."""
+    tokens, hidden, topk, experts = 37, 256, 2, 8
+    cfg = Config(hidden_size=hidden, topk=topk, max_tokens_per_rank=tokens, timeout_seconds=2.0)
+    with EmulatedGroup(1, [0] * experts, cfg) as group:
+        slot, dev = group.create_slot(), group.device
+        x = torch.zeros((tokens, hidden), dtype=torch.bfloat16, device=dev)
+        ids = torch.zeros((tokens, topk), dtype=torch.int64, device=dev)
+        weights = torch.zeros((tokens, topk), device=dev)
+        out, other = torch.empty_like(x), torch.zeros(1, device=dev)
+        main, side = torch.cuda.Stream(), torch.cuda.Stream()
+
+        def layer():
+            batch = group.dispatch(slot, [x], [ids], [weights], stream=main)[0]
+            side.wait_stream(main)
+            partial = group.scale_rows(batch, stream=side)
+            with torch.cuda.stream(main):
+                other.add_(1)                                   # runs beside the expert
+            main.wait_stream(side)
+            group.combine(slot, [partial], [tokens], outs=[out], stream=main)
+
+        ids.copy_(workloads.uniform_routing(tokens, experts, topk, seed=0, rank=0)[0])
+        torch.cuda.synchronize()
+        layer()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=main):
+            layer()
+        for seed in range(3):
+            i, w = workloads.uniform_routing(tokens, experts, topk, seed=seed, rank=0)
+            payload = workloads.gaussian_payload(tokens, hidden, seed=seed, rank=0)
+            ids.copy_(i), weights.copy_(w), x.copy_(payload)
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            plan = routing.plan_routes([i], [w], [0] * experts, 1, topk)
+            want = routing.combine_oracle(expected_partials(plan, [payload], None), plan, hidden, "two_step")
+            assert torch.equal(bits(out), bits(want[0]))
+        assert group.status()[0][0] == 0
+
+
 def test_intermediate_rounding_is_observable():
     """remote-sum -> bf16 -> + local -> bf16 differs from a single rounding on chosen values."""
     world, hidden = 3, 64
