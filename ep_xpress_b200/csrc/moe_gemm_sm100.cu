@@ -414,6 +414,10 @@ constexpr int kAlignThreads = 1024;
 constexpr int kMaxLocalExperts = 1024;
 constexpr int kAlignClusterMax = 8;
 
+// Rows to work on: the device's count bounded to [0, rows]. A negative count is an empty batch: as an
+// unsigned number of a mover's items it would be four billion of them.
+__device__ __forceinline__ int usable_rows(int valid_count, int rows) { return max(0, min(valid_count, rows)); }
+
 // Exclusive prefix sum over the CTA's 1024 threads (`warp_sums` is 32 words of shared memory).
 __device__ __forceinline__ int warp_inclusive_scan(int v, int lane) {
 #pragma unroll
@@ -461,7 +465,7 @@ __global__ void __launch_bounds__(kAlignThreads) moe_align_kernel(const long lon
   __syncthreads();
   wait_for_previous();
   launch_dependents();
-  const int pairs = min(*valid_count, rows) * topk;
+  const int pairs = usable_rows(*valid_count, rows) * topk;
   const int step = static_cast<int>(ctas) * kAlignThreads;
   constexpr int kBatch = 4;                          // independent loads in flight per thread
   // The first batch of a thread stays in registers between the two passes, weights included; up to
@@ -568,7 +572,7 @@ __global__ void __launch_bounds__(256) moe_scatter_kernel(const uint4* __restric
   launch_dependents();
   const int lane = threadIdx.x & 31;
   const unsigned units = units_per_row(vecs_per_row);
-  const unsigned items = min(*valid_count, rows) * units;
+  const unsigned items = usable_rows(*valid_count, rows) * units;
   const unsigned warps = gridDim.x * (blockDim.x / 32);
   for (unsigned item = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); item < items; item += warps) {
     const unsigned row = item / units;
@@ -604,7 +608,7 @@ __global__ void __launch_bounds__(256) moe_slot_sum_kernel(const uint4* __restri
   launch_dependents();
   const int lane = threadIdx.x & 31;
   const unsigned units = (vecs_per_row + 32 * kVecs - 1) / (32 * kVecs);
-  const unsigned items = min(*valid_count, rows) * units;
+  const unsigned items = usable_rows(*valid_count, rows) * units;
   const unsigned warps = gridDim.x * (blockDim.x / 32);
   for (unsigned item = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); item < items; item += warps) {
     const unsigned row = item / units;

@@ -131,6 +131,18 @@ def test_token_tile_edges_match_fp32_reference(counts, pad, gather_loads):
     assert (out[valid:] == 7.0).all()
 
 
+@pytest.mark.parametrize("count", [-1, -(2 ** 31)])
+@pytest.mark.parametrize("rows,gather_loads", [(5, False), (5, True), (10000, False)])     # both forms of the slot sum
+def test_negative_count_is_an_empty_batch(rows, gather_loads, count):
+    """The count is a device value that no host check sees: nothing is read or written for it."""
+    x, ids, weights, _, w13, w2 = make_case(rows, 2, 2, 256, 128, rows, seed=11)
+    runner = GroupedSwiGLU(w13, w2, max_rows=rows, topk=2, gather_loads=gather_loads)
+    out = torch.full_like(x, 7.0)
+    runner(x, ids, weights, torch.tensor([count], dtype=torch.int32, device="cuda"), out=out)
+    runner.check()
+    assert (out == 7.0).all() and runner.counters.tolist() == [0, 0]
+
+
 def test_pair_bound_overflow_is_reported():
     x, ids, weights, count, w13, w2 = make_case(512, 4, 2, 256, 128, 512, seed=3, local_fraction=1.0)
     runner = GroupedSwiGLU(w13, w2, max_rows=512, topk=4, max_local_pairs=128)
