@@ -685,9 +685,8 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_kernel(const __grid_cons
 // a few CTAs, a rank-wide barrier, the tile prefix, claims from a counter - is most of its distance
 // from the copy bound. Here CTA c owns tokens [T c / ctas, T (c + 1) / ctas): it routes them, its
 // movers start to load, and it publishes how many of them are live as one tagged word and sums the
-// words of all CTAs (one round trip, hidden under the loads). A batch of at most 768 tokens is routed
-// by every CTA and needs no exchange and no cooperative launch (hidden 2048, dispatch + expert + combine
-// of 600 tokens: 14.4 us, 17.3 with the exchange); 1024 tokens cost more that way (18.5 us against 17.7).
+// words of all CTAs (one round trip, hidden under the loads). A small batch is routed by every CTA and
+// needs no exchange and no cooperative launch (see lone_solo for the line).
 // The payload is bound by HBM (or L2): eight movers with a ring of three 7 KB pieces each keep 172 KB
 // per SM in flight, and a stage is refilled as soon as its own store has read it. Kernel time, one
 // rank, hidden 7168: 128 tokens 8 -> 5.3 us, 4096 tokens 37 -> 27 us.
@@ -698,7 +697,7 @@ constexpr int kEarlyStages = 1;
 constexpr size_t kLoneSmemBytes = static_cast<size_t>(kLoneMovers) * kLoneStages * kLonePieceBytes;
 constexpr int kMetaThreads = kThreads - 32 * kLoneMovers;
 constexpr int kLoneMaxCtas = 512;
-constexpr int kSoloTokens = 768;          // batches that every CTA routes for itself
+constexpr int kSoloTokens = 768;          // largest batch that every CTA routes for itself
 constexpr unsigned kLoneTag = 0x80000000u;   // no generation and no row position has this bit
 
 struct LoneDispatchArgs {
@@ -706,6 +705,7 @@ struct LoneDispatchArgs {
   RankCtx ctx;
   char* heap;
   SlotLayout layout;
+  bool solo;                              // every CTA routes the whole batch (at most kSoloTokens)
 };
 
 // All but the `kLeft` youngest bulk-copy groups of this thread have read their source.
@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
   if (!ok && tid == 0 && cta == 0) report_error(c, kEpochsExhausted, kPhaseDispatch, 0xE0, g);
   const unsigned sample = ok ? sample_begin(op.samples, g, op.sample_capacity) : ~0u;
   // Tokens this CTA routes: all of a small batch, else its own.
-  const bool solo = T <= kSoloTokens;
+  const bool solo = args.solo;
   const int route_first = solo ? 0 : first, route_count = solo ? T : mine;
   const int route_words = solo ? kSoloTokens / 32 : kWarps;
   for (int i = tid; i < route_words * 32; i += kThreads) {
@@ -1022,27 +1022,42 @@ cudaError_t dispatch_max_ctas(bool ids64, bool vec16, size_t dynamic_smem, int* 
   return cudaSuccess;
 }
 
+// Whether every CTA of a one-rank dispatch routes the whole batch itself. Up to kRegK slots a route is
+// one round trip of independent loads: 768 tokens against 769, hidden 2048 / 7168, top-8, us of dispatch
+// + combine: 11.6 / 13.4 against 12.2 / 14.9 with the exchange (1024 tokens: 18.5 a layer pass solo, 17.7
+// exchanged). Above kRegK it is a serial loop over slot pairs that costs more with every token a CTA has
+// (hidden 2048, solo against exchanged: top-12, 128 / 512 tokens 12.6 / 20.3 against 12.8 / 15.7; top-16,
+// 4 / 32 / 512 tokens 13.1 / 17.5 / 47 against 12.9 / 13.1 / 17.5; top-32, 512 tokens 156 against 26).
+// Where the slot has no room for the exchange's words, a batch of one token per thread is routed solo.
+static bool lone_solo(const DispatchOp& op, int topk, bool words_fit) {
+  const int line = topk <= kRegK ? kSoloTokens : (topk <= 12 ? 256 : 4);
+  return op.tokens <= line || (!words_fit && op.tokens <= kThreads);
+}
+
 // A group of one rank takes its own kernel, except where that kernel's plan does not hold: rows that
 // are not 16-byte aligned (bulk copies), profiled operations (phase stamps of the general kernel),
 // more than 512 tokens per CTA (one thread routes one), and slots too small for the count words.
-static bool lone_applies(const DispatchArgs& args, int ranks, int world, int ctas, bool vec16) {
+static bool lone_applies(const DispatchArgs& args, int ranks, const RankCtx& host_ctx, int ctas, bool vec16, bool* solo) {
   const DispatchOp& op = args.op[0];
-  if (world != 1 || ranks != 1 || !vec16 || op.profile != nullptr || ctas > kLoneMaxCtas) return false;
+  if (host_ctx.world != 1 || ranks != 1 || !vec16 || op.profile != nullptr || ctas > kLoneMaxCtas) return false;
   if (op.tokens > static_cast<long long>(ctas) * kThreads) return false;
-  return op.tokens <= kSoloTokens || 2 * ctas <= op.slot_tokens;
+  const bool words_fit = 2 * ctas <= op.slot_tokens;
+  *solo = lone_solo(op, host_ctx.topk, words_fit);
+  return *solo || words_fit;
 }
 
 cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, const RankCtx& host_ctx, int ctas_per_rank, bool ids64,
                             bool vec16, size_t dynamic_smem, bool cooperative, cudaStream_t stream) {
-  if (lone_applies(args, ranks, host_ctx.world, ctas_per_rank, vec16)) {
-    LoneDispatchArgs lone_args{args.op[0], host_ctx, host_ctx.heap[host_ctx.rank], {}};
+  bool solo = false;
+  if (lone_applies(args, ranks, host_ctx, ctas_per_rank, vec16, &solo)) {
+    LoneDispatchArgs lone_args{args.op[0], host_ctx, host_ctx.heap[host_ctx.rank], {}, solo};
     lone_args.layout = slot_layout(args.op[0].slot_capacity, args.op[0].slot_tokens, host_ctx.hidden, host_ctx.topk, 1);
     const auto lone = ids64 ? dispatch_lone_kernel<long long> : dispatch_lone_kernel<int>;
     cudaError_t err = cudaFuncSetAttribute(lone, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLoneSmemBytes));
     if (err != cudaSuccess) return err;
     void* lone_params[] = {&lone_args};
     // A batch that every CTA routes itself has no CTA waiting for another: a plain launch is enough.
-    if (!cooperative || args.op[0].tokens <= kSoloTokens)
+    if (!cooperative || solo)
       return cudaLaunchKernel(reinterpret_cast<const void*>(lone), dim3(ctas_per_rank, 1, 1), dim3(kThreads, 1, 1),
                               lone_params, kLoneSmemBytes, stream);
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(lone), dim3(ctas_per_rank, 1, 1),

@@ -146,9 +146,12 @@ def test_one_rank_group_streams_local_rows(hidden, tokens, rounding):
 @pytest.mark.parametrize("tokens,hidden,topk,ctas", [
     (1, 64, 2, 1), (512, 264, 8, 3), (513, 264, 8, 3), (600, 3592, 3, 2), (1021, 3584, 9, 148), (700, 258, 4, 7),
     (768, 64, 8, 5), (769, 64, 8, 5), (1030, 3592, 3, 2),
+    (256, 64, 9, 2), (257, 264, 9, 2), (4, 64, 13, 2), (5, 64, 13, 2), (768, 264, 16, 148),
+    (64, 64, 16, 40),
 ])
 def test_one_rank_dispatch_at_the_edges_of_its_plan(tokens, hidden, topk, ctas):
-    """Batches routed by every CTA (up to 768 tokens) and by shares, one and several pieces per row,
+    """Batches routed by every CTA (up to 768 tokens, fewer above eight slots) and by shares, slots without
+    room for the shares' words, one and several pieces per row,
     rows the bulk copies cannot take, tokens without a route, a smaller batch after a larger one."""
     cfg = Config(hidden_size=hidden, topk=topk, max_tokens_per_rank=tokens, timeout_seconds=2.0)
     emap = workloads.round_robin_expert_map(16, 1)
