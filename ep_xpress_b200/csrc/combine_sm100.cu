@@ -707,16 +707,40 @@ __device__ __forceinline__ bool mailbox_push(const PushArgs& p, const RankCtx& c
   return fine;
 }
 
+// Stores the arrival words of rows that other warps of this CTA know to be complete at their owners:
+// `count` word addresses (0: none) in shared memory, behind the barrier that follows those warps' stores
+// or acquires. Called by ONE warp. Every lane fences before it stores: a fence orders what it sees only
+// before the stores of the thread that ran it, so a fence in one thread and the words in others, with a
+// barrier between them, is not a release at system scope. The fence is cumulative over the other warps'
+// rows through the barrier; 32 lanes run it as one instruction. The first kHeld words of a lane wait for
+// the fence in registers.
+template <int kHeld, bool kProfile>
+__device__ __forceinline__ void publish_words(const unsigned long long* words, int count, unsigned epoch, int lane,
+                                              Profiler<kProfile>& prof) {
+  unsigned long long held[kHeld];
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) held[i] = i * 32 + lane < count ? words[i * 32 + lane] : 0ull;
+  __threadfence_system();
+  auto store = [&](unsigned long long word) {
+    if (word == 0ull) return;
+    st_relaxed_sys_u32(reinterpret_cast<unsigned*>(word), epoch);
+    prof.first(kProfFirstPublish);
+  };
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) store(held[i]);
+  for (int i = kHeld * 32 + lane; i < count; i += 32) store(words[i]);
+}
+
 // The herald warps of a herald CTA, one per pusher, on an SM whose only stores are arrival words. Whenever
-// some pushers have posted rounds: ONE system-scope fence for the CTA - cumulative over those pushers'
-// completed copies, which reached its warps through the release/acquire on `posted` and then the
-// barrier - and every warp stores its pusher's arrival words relaxed (lane l: the word of stage l). A
-// release per word would serialise a round trip to the peer per word, and a fence per warp queues up
-// sixteen fences on the SM: the last words left 20 us after the last row. Called by all threads of the
-// CTA; `slot` is null in warps without a pusher.
+// some pushers have posted rounds, their warps collect the rounds' word addresses in shared memory
+// (lane l: the word of stage l) and ONE warp publishes them all behind one system-scope fence. A release
+// per word would serialise a round trip to the peer per word, and a fence per warp queues up sixteen
+// fences on the SM: the last words left 20 us after the last row. Called by all threads of the CTA;
+// `slot` is null in warps without a pusher. `words` holds kHeraldWords addresses.
+constexpr int kHeraldWords = kHeraldWarpsPerCta * kPushSlotRounds * kPushRoundWords;
 template <bool kProfile>
-__device__ __forceinline__ bool mailbox_herald(const RankCtx& c, PushSlot* slot, unsigned epoch, int lane,
-                                               Profiler<kProfile>& prof) {
+__device__ __forceinline__ bool mailbox_herald(const RankCtx& c, PushSlot* slot, unsigned epoch,
+                                               unsigned long long* words, int warp, int lane, Profiler<kProfile>& prof) {
   unsigned done = 0;                                      // rounds whose words are out
   const unsigned long long start = global_timer_ns();
   unsigned spins = 0;
@@ -724,20 +748,20 @@ __device__ __forceinline__ bool mailbox_herald(const RankCtx& c, PushSlot* slot,
     unsigned long long both = 0;
     // (posted, final_rounds) in one load; a pusher that is done posts nothing more.
     if (lane == 0 && slot != nullptr) both = ld_acquire_gpu_u64(reinterpret_cast<const unsigned long long*>(&slot->posted));
+    __syncwarp();                                         // the other lanes read words behind lane 0's acquire
     both = __shfl_sync(0xffffffffu, both, 0);
     const unsigned posted = static_cast<unsigned>(both), final_rounds = static_cast<unsigned>(both >> 32);
+    // A pusher is never more than kPushSlotRounds rounds ahead of `heralded`. Warps without news clear
+    // their part: it may hold the words of an earlier turn.
+    if (warp < kHeraldWarpsPerCta && lane < kPushRoundWords) {
+#pragma unroll
+      for (unsigned i = 0; i < kPushSlotRounds; ++i)
+        words[(i * kHeraldWarpsPerCta + warp) * kPushRoundWords + lane] =
+            done + i < posted ? ld_relaxed_sys(&slot->words[(done + i) % kPushSlotRounds][lane]) : 0ull;
+    }
     if (__syncthreads_or(posted != done)) {
-      if (threadIdx.x == 0) __threadfence_system();
-      __syncthreads();
-      for (unsigned round = done; round != posted; ++round) {
-        unsigned long long word = 0;
-        if (lane < kPushRoundWords) word = ld_relaxed_sys(&slot->words[round % kPushSlotRounds][lane]);
-        if (word != 0ull) {
-          st_relaxed_sys_u32(reinterpret_cast<unsigned*>(word), epoch);
-          prof.first(kProfFirstPublish);
-        }
-      }
-      __syncwarp();
+      if (warp == 0) publish_words<kHeraldWarpsPerCta * kPushRoundWords / 32, kProfile>(words, kHeraldWords, epoch, lane, prof);
+      __syncthreads();                                    // the words are read before they are written again
       if (lane == 0 && posted != done) st_release_gpu_u32(&slot->heralded, posted);
       done = posted;
       continue;
@@ -753,16 +777,22 @@ __device__ __forceinline__ bool mailbox_herald(const RankCtx& c, PushSlot* slot,
 
 // ---- mailbox push, small batches -------------------------------------------------------------
 // One round per pusher warp and nothing to overlap: what counts is the length of the chain. Every warp
-// of a push CTA moves whole rows through registers (look-up, loads, peer stores), one system-scope
-// fence orders two rows of every warp before their arrival words, so a CTA has 24 rows under way where the bulk-copy pusher has fifteen and a
-// copy through shared memory between each load and store; and it takes them from the received rows
-// themselves (the other ranks' rows, starting behind this rank's own), without holes and claims.
+// of a push CTA moves whole rows through registers (look-up, loads, peer stores) and one warp publishes
+// two rows of every warp behind one system-scope fence (an SM runs its warps' fences one after the
+// other), so a CTA has 24 rows under way where the bulk-copy pusher has fifteen and a copy through shared
+// memory between each load and store; and it takes them from the received rows themselves (the other
+// ranks' rows, starting behind this rank's own), without holes and claims. `words` is shared memory for
+// two times kRows addresses per warp of the CTA: one warp publishes a turn's while the others, which it
+// meets at the next barrier, write the next turn's.
 template <bool kProfile>
 __device__ __forceinline__ void mailbox_push_rows(const PushArgs& p, unsigned epoch, int received, int warp, int warps,
-                                                  int lane, Profiler<kProfile>& prof) {
+                                                  unsigned long long* words, int lane, Profiler<kProfile>& prof) {
   constexpr int kUnroll = 10;
   constexpr int kRows = 2;             // rows of a warp per fence
+  constexpr int kWords = kRows * (kMailThreads / 32);
+  const int cta_warp = static_cast<int>(threadIdx.x >> 5);
   const int own = p.rows_from[p.self], after_own = p.first_row[p.self] + own, count = received - own;
+  int turn = 0;
   for (int begin = 0; begin < count; begin += kRows * warps) {        // the same trips for every warp
     char* moved[kRows];
 #pragma unroll
@@ -789,18 +819,16 @@ __device__ __forceinline__ void mailbox_push_rows(const PushArgs& p, unsigned ep
           if (base + u * 512 < p.row_bytes) store_chunk<4>(dst + base + u * 512, v[u]);
       }
     }
-    // One fence for the CTA's rows, cumulative through the barrier: an SM runs its warps' system-scope
-    // fences one after the other.
-    __syncthreads();
-    if (threadIdx.x == 0) __threadfence_system();
-    __syncthreads();
+    if (lane == 0) {
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
-      if (moved[j] == nullptr || lane != 0) continue;
-      st_relaxed_sys_u32(reinterpret_cast<unsigned*>(moved[j] + p.row_bytes), epoch);
-      prof.first(kProfFirstPublish);
-      prof.moved(1, static_cast<unsigned long long>(p.row_bytes));
+      for (int j = 0; j < kRows; ++j) {
+        words[turn * kWords + cta_warp * kRows + j] = moved[j] != nullptr ? reinterpret_cast<unsigned long long>(moved[j] + p.row_bytes) : 0ull;
+        if (moved[j] != nullptr) prof.moved(1, static_cast<unsigned long long>(p.row_bytes));
+      }
     }
+    __syncthreads();
+    if (cta_warp == 0) publish_words<(kWords + 31) / 32, kProfile>(words + turn * kWords, kWords, epoch, lane, prof);
+    turn ^= 1;
   }
 }
 
@@ -1029,7 +1057,8 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
     debug_delay(c, 4);
     if (cta < push_ctas) {
       if (op.herald == 0) {
-        mailbox_push_rows<kProfile>(push, e, s_received, cta + (tid >> 5) * push_ctas, push_ctas * (kMailThreads / 32), lane, prof);
+        mailbox_push_rows<kProfile>(push, e, s_received, cta + (tid >> 5) * push_ctas, push_ctas * (kMailThreads / 32),
+                                    reinterpret_cast<unsigned long long*>(dynamic_smem), lane, prof);
       } else if (tid < 32) {
         if (!mailbox_push<kProfile>(push, c, hdr, dynamic_smem, s_push_full, e, heralds ? hand + cta : nullptr, lane,
                                     push_ctas, prof) && lane == 0)
@@ -1039,7 +1068,8 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
     } else if (cta < push_ctas + herald_ctas) {
       const int pusher = (cta - push_ctas) * kHeraldWarpsPerCta + (tid >> 5);
       const bool owner = (tid >> 5) < kHeraldWarpsPerCta && pusher < push_ctas;
-      if (!mailbox_herald<kProfile>(c, owner ? hand + pusher : nullptr, e, lane, prof) && lane == 0)
+      if (!mailbox_herald<kProfile>(c, owner ? hand + pusher : nullptr, e, reinterpret_cast<unsigned long long*>(dynamic_smem),
+                                    tid >> 5, lane, prof) && lane == 0)
         report_error(c, kTimeout, kPhaseCombine, 8, 0);
     } else {
       reduce.cta = cta - push_ctas - herald_ctas;

@@ -298,6 +298,27 @@ def test_both_combine_protocols_match_the_oracle(world, hidden, topk, tokens, ct
                       rounding="two_step")
 
 
+@pytest.mark.parametrize("world,hidden,topk,tokens,ctas", [
+    (2, 64, 2, 1, 2), (2, 64, 2, 49, 2),      # one push CTA: a single row, more rows than one fence covers
+    (3, 512, 3, 640, None),                   # the largest slot pushed through registers (1920 rows)
+    (3, 512, 3, 641, None),                   # the smallest with heralds: 21 pushers, a full and a partial herald CTA
+    (2, 64, 2, 2000, 74),                     # two full herald CTAs, several rounds per pusher
+    (2, 256, 2, 1000, 4), (2, 256, 2, 1000, 3),   # the smallest launch with a herald CTA; pushers that publish themselves
+])
+def test_arrival_words_leave_through_one_warp(world, hidden, topk, tokens, ctas):
+    """Who fences and stores the arrival words, at the sizes where that changes; with and without delays."""
+    emap = workloads.round_robin_expert_map(world * 2, world)
+    for delay in (0, 3000):
+        cfg = Config(hidden_size=hidden, topk=topk, max_tokens_per_rank=tokens, timeout_seconds=2.0, debug_delay_ns=delay)
+        with EmulatedGroup(world, emap, cfg) as group:
+            slot = group.create_slot()
+            for seed in range(3):
+                n = [tokens if seed != 1 else max(tokens - 7 * rank, 0) for rank in range(world)]
+                routes = [workloads.uniform_routing(n[r], world * 2, topk, seed=seed, rank=r) for r in range(world)]
+                xs = [workloads.gaussian_payload(n[r], hidden, seed=seed, rank=r) for r in range(world)]
+                run_round(group, slot, xs, [i for i, _ in routes], [w for _, w in routes], emap, ctas=ctas)
+
+
 def test_a_short_partial_is_an_error_not_stale_data():
     """A rank whose partial tensor has fewer rows than it received cannot serve every owner: it
     reports a capacity error and the owners that wait for the missing rows stop with a status,
