@@ -606,6 +606,7 @@ __device__ __forceinline__ bool mailbox_push(const PushArgs& p, const RankCtx& c
   auto publish = [&]() -> bool {
     bulk_wait_all_complete();
     fence_proxy_async();               // the copies wrote through the async proxy; the words below are ordinary stores
+    __syncwarp();                      // the lane that publishes a row is not the one that moved its first pieces
     unsigned* const word = pending;
     pending = nullptr;
     // A round that only met holes of the interleaved order completed no row: nothing to order,
@@ -917,6 +918,7 @@ __device__ __forceinline__ bool mailbox_reduce(const BulkReduceArgs& a, const Ra
       }
     }
     if (!__all_sync(0xffffffffu, fine)) return false;
+    __syncwarp();        // all lanes read the rows that lane j's acquire covers; a vote alone orders no memory
     if (lane == 0) prof.count(kProfItems, 1);
     const unsigned valid = __ballot_sync(0xffffffffu, src != nullptr);
     const unsigned vote = __ballot_sync(0xffffffffu, is_self);
