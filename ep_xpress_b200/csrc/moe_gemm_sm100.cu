@@ -175,6 +175,14 @@ struct GemmMaps {
   CUtensorMap b[kNMaps];         // the token matrix with boxes of 8 << i rows
 };
 
+// Token tile `index` of the list that the align step wrote. Acquiring loads: they go to L2, so that a kernel
+// that has not waited for the one before it yet never takes a stale line of the SM's L1 for the list.
+__device__ __forceinline__ int4 acquire_tile(const int4* tiles, int index) {
+  const unsigned long long* p = reinterpret_cast<const unsigned long long*>(tiles + index);
+  const unsigned long long low = ld_acquire_gpu_u64(p), high = ld_acquire_gpu_u64(p + 1);
+  return make_int4(static_cast<int>(low), static_cast<int>(low >> 32), static_cast<int>(high), static_cast<int>(high >> 32));
+}
+
 // Index of the smallest box that holds `half` token rows (a multiple of 8).
 __device__ __forceinline__ int box_index(int half) {
   return half <= 8 ? 0 : (half <= 16 ? 1 : (half <= 32 ? 2 : (half <= 64 ? 3 : 4)));
@@ -239,12 +247,13 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
   // The tile list comes from the align step, which is complete before the launch right behind it lets
   // this kernel start; only the tokens (and, when gathered, the list itself) are the previous kernel's.
   // So the producer fills its ring with the first tile's WEIGHTS while the previous kernel ends, and
-  // waits before the first token load. Every thread waits before it leaves.
+  // waits before the first token load; it reads the list with acquiring loads until then. (One thread of
+  // warp 0 waits in that mode, all threads of the other warps do, and the CTA leaves behind them all.)
   if (p.gather_rows != nullptr || warp != 0) {
     wait_for_previous();
     launch_dependents();
   }
-  const int total = p.counters[0] * p.m_tiles;
+  const int total = static_cast<int>(ld_acquire_gpu_u32(reinterpret_cast<const unsigned*>(p.counters))) * p.m_tiles;
   const int pair_id = blockIdx.x / 2, pairs = gridDim.x / 2;
 
   auto load_weights = [&](unsigned char* dst, int k, int expert, int mt, unsigned leader_full) {
@@ -291,7 +300,7 @@ grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
       int ahead = 0;                                 // k-steps of the first tile whose weights are under way
       if (pair_id < total) {
         const int tt = pair_id / p.m_tiles, mt = pair_id - tt * p.m_tiles;
-        const int4 tile = p.tiles[tt];
+        const int4 tile = acquire_tile(p.tiles, tt);
         const unsigned tx = 2u * (kABytes + (8u << box_index(((tile.z + 15) & ~15) / 2)) * kTileK * 2);
         for (; ahead < stages && ahead < p.k_steps; ++ahead) {
           if (rank == 0) mbarrier_arrive_expect_tx(full_bar + ahead, tx);
