@@ -86,6 +86,37 @@ def run_replay(ep, rank, world, args):
     ep.check()
 
 
+def run_strided(ep, rank, world, args):
+    """Ids and weights that are strided views, written behind a long kernel on a stream that is not current:
+    the copies that make them contiguous are ordered behind it, for tickets and for direct calls."""
+    hidden, topk, tokens = args.hidden, 4, args.tokens
+    emap = workloads.contiguous_expert_map(world * 4, world)
+    factors = [torch.ones(4) for _ in range(world)]
+    side = torch.cuda.Stream()
+    wide_ids = torch.full((tokens, topk + 3), -1, dtype=torch.int64, device="cuda")
+    wide_weights = torch.zeros((tokens, topk + 1), device="cuda")
+    torch.cuda.synchronize()
+    for iteration in range(0, 8, 2):                            # even iterations: every rank has all its tokens
+        xs, ids, ws = group_inputs("uniform", world, tokens, hidden, topk, iteration)
+        plan, rows, want = expected(xs, ids, ws, emap, world, topk, hidden, factors)
+        x, i, w = xs[rank].cuda(), ids[rank].cuda(), ws[rank].cuda()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)
+            wide_ids[:, 1:1 + topk].copy_(i)
+            wide_weights[:, 1:].copy_(w)
+        strided = (x, wide_ids[:, 1:1 + topk], wide_weights[:, 1:])
+        if iteration % 4:
+            batch = ep.dispatch_on_stream(*strided, stream=side)
+            torch.cuda.current_stream().wait_stream(side)
+        else:
+            batch = ep.dispatch_async(*strided, stream=side).wait()
+        check_batch(batch, plan, rows, rank)
+        out = ep.combine_on_stream(scale_rows(ep, batch), batch.handle)
+        assert torch.equal(bits(out), bits(want[rank]))
+    ep.check()
+
+
 def run_reverse_handles(ep, rank, world, args):
     """Two dispatches outstanding, combined in reverse (rank-consistent) order."""
     hidden, topk, tokens = args.hidden, 4, args.tokens
@@ -512,7 +543,7 @@ def run_profile(ep, rank, world, args):
     ep.check()
 
 
-CASES = {"streams": run_streams, "stagger": run_stagger, "headline": run_headline, "profile": run_profile, "replay": run_replay, "reverse": run_reverse_handles, "graph": run_graph, "errors": run_errors}
+CASES = {"streams": run_streams, "stagger": run_stagger, "headline": run_headline, "profile": run_profile, "replay": run_replay, "strided": run_strided, "reverse": run_reverse_handles, "graph": run_graph, "errors": run_errors}
 
 
 def main():

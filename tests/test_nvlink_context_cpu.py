@@ -101,6 +101,48 @@ def test_direct_dispatch_plumbs_arguments_and_emits_no_ticket(ctx):
         ctx.ep.combine_on_stream(torch.zeros(12, 16, dtype=torch.bfloat16), batch.handle)
 
 
+@pytest.mark.parametrize("asynchronous", [True, False])
+@pytest.mark.parametrize("explicit", [True, False])
+def test_inputs_are_copied_on_the_stream_that_reads_them(ctx, asynchronous, explicit):
+    """Strided ids and weights and a misaligned payload are copied behind the waits of the executing stream, on
+    that stream, whatever stream is current; the caller's tensors stay alive for a stream that is not theirs."""
+    log, entered, side = [], [ctx.main], FakeStream("side")
+
+    @contextlib.contextmanager
+    def scope(stream):
+        entered.append(stream)
+        yield
+        entered.pop()
+
+    def logged(name):
+        original = getattr(torch.Tensor, name)
+
+        def call(tensor, *args, **kwargs):
+            log.append((name, entered[-1].name, tuple(ctx.ep._work_stream.waits)))
+            return original(tensor, *args, **kwargs)
+        return call
+
+    recorded = []
+    x = torch.arange(1 + 4 * 16, dtype=torch.float32).to(torch.bfloat16)[1:].view(4, 16)
+    ids, weights = torch.arange(16).view(4, 4)[:, :2], torch.rand(4, 4)[:, 1:3]
+    assert x.data_ptr() % 4 and not ids.is_contiguous() and not weights.is_contiguous()
+    with mock.patch.object(torch.cuda, "stream", scope), \
+            mock.patch.object(torch.Tensor, "record_stream", lambda t, s: recorded.append((id(t), s.name))), \
+            mock.patch.object(torch.Tensor, "contiguous", logged("contiguous")), \
+            mock.patch.object(torch.Tensor, "clone", logged("clone")):
+        submit = ctx.ep.dispatch_async if asynchronous else ctx.ep.dispatch_on_stream
+        submit(x, ids, weights, stream=side if explicit else None)
+    producer = "side" if explicit else "main"
+    reader = "work" if asynchronous else producer
+    assert [(name, stream) for name, stream, _ in log] == [("contiguous", reader)] * 2 + [("clone", reader)]
+    if asynchronous:
+        assert all(producer in waits for _, _, waits in log)
+        assert set(recorded) >= {(id(t), "work") for t in (x, ids, weights)}
+    got = [tensors[0] for tensors in ctx.core.dispatch.call_args[0][1:4]]
+    assert all(t.is_contiguous() for t in got) and got[0].data_ptr() % 4 == 0
+    assert all(torch.equal(a, b) for a, b in zip(got, (x, ids, weights)))
+
+
 def test_diagnostics_hashes_phase_tag_and_operation(ctx):
     object.__setattr__(ctx.ep.config, "diagnostics", True)
     batch = ctx.ep.dispatch_on_stream(*inputs(), tag="a")

@@ -9,6 +9,6 @@ from test_nvlink_multigpu import launch
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(gpu_count() < 1, reason="needs a CUDA device")]
 
 
-@pytest.mark.parametrize("case", ["replay", "graph", "profile", "reverse"])
+@pytest.mark.parametrize("case", ["replay", "graph", "profile", "reverse", "strided"])
 def test_one_rank_group(case):
     launch(case, 1)
