@@ -143,6 +143,17 @@ def test_inputs_are_copied_on_the_stream_that_reads_them(ctx, asynchronous, expl
     assert all(torch.equal(a, b) for a, b in zip(got, (x, ids, weights)))
 
 
+def test_batches_of_a_pool_slot_are_the_callers_own(ctx):
+    """What a caller does to its batch's tensor objects does not reach the next operation of the slot."""
+    first = ctx.ep.dispatch_on_stream(*inputs())
+    first.hidden.unsqueeze_(0), first.local_ids.t_(), first.weights.unsqueeze_(-1), first.handle.inverse_map.t_()
+    ctx.ep.combine_on_stream(torch.zeros(16, 16, dtype=torch.bfloat16), first.handle)
+    batch = ctx.ep.dispatch_on_stream(*inputs())
+    assert batch.handle._plan.slot is first.handle._plan.slot
+    assert batch.hidden.shape == (16, 16) and batch.local_ids.shape == (16, 2) and batch.weights.shape == (16, 2)
+    assert batch.handle.inverse_map.shape == (16, 2)
+
+
 def test_diagnostics_hashes_phase_tag_and_operation(ctx):
     object.__setattr__(ctx.ep.config, "diagnostics", True)
     batch = ctx.ep.dispatch_on_stream(*inputs(), tag="a")
