@@ -878,9 +878,10 @@ __device__ __forceinline__ void mailbox_add(const char* staged, long long stride
 template <bool kProfile>
 __device__ __forceinline__ bool mailbox_reduce(const BulkReduceArgs& a, const RankCtx& c, unsigned epoch, int warp,
                                                int warps, int lane, Profiler<kProfile>& prof) {
-  // 2 KB segments, cut to what one round of loads covers (eight rows' worth of 512 bytes) while that
-  // leaves warps without an item.
-  int seg = 2048;
+  // 2 KB segments, 4 KB where a token has one contributor (eight loads per lane in flight; with 2 KB
+  // there were four: 4 x 1024 x 7168, top-1, 62.8 -> 51.6 us), cut towards one round of loads (eight
+  // rows' worth of 512 bytes) while that leaves warps without an item.
+  int seg = a.fan <= 1 ? 4096 : 2048;
   const int round = a.fan <= 2 ? 2048 : (a.fan <= 4 ? 1024 : 512);
   const long long workers = static_cast<long long>(a.ctas) * warps;
   while (seg > round && a.tokens * ((a.row_bytes + seg - 1) / seg) < 2 * workers) seg /= 2;
@@ -927,7 +928,8 @@ __device__ __forceinline__ bool mailbox_reduce(const BulkReduceArgs& a, const Ra
     const char* const local = reinterpret_cast<const char*>(local_bits);
     const char* const staged = a.staging + t * a.fan * a.stride;
     char* const outp = a.out + t * a.row_bytes;
-    if (n <= 2) mailbox_add<2, 4>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
+    if (n <= 1) mailbox_add<1, 8>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
+    else if (n <= 2) mailbox_add<2, 4>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
     else if (n <= 4) mailbox_add<4, 2>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
     else mailbox_add<8, 1>(staged, a.stride, local, valid, self_index, outp, b0, b1, lane, a.single_round);
   }

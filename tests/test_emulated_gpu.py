@@ -275,6 +275,7 @@ def test_invalid_routes_are_reported():
     (4, 264, 4, 33, None),        # rows that are not 16-byte multiples: the register path runs instead
     (2, 8192, 2, 40, 7),          # rows larger than one mover / pusher stage: two pieces per row
     (2, 8192, 2, 1000, 9),        # the same with heralds and several rounds per pusher
+    (4, 2056, 1, 150, None), (2, 3592, 1, 700, 5), (3, 64, 1, 40, None),   # one contributor per token: 4 KB segments
 ])
 def test_both_combine_protocols_match_the_oracle(world, hidden, topk, tokens, ctas, protocol):
     """Mailbox (push and reduce side by side, one arrival word per row) and sequential (push,
