@@ -1054,13 +1054,13 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
     // ---- push CTAs, herald CTAs and reduce CTAs side by side ----
     // (A mailbox launch has at least two CTAs; heralds are used from kMinHeraldLaunch CTAs on.)
     const int push_ctas = mailbox_push_ctas(static_cast<int>(gridDim.x));
-    const bool heralds = op.herald != 0 && static_cast<int>(gridDim.x) >= kMinHeraldLaunch + 1;
+    const bool heralds = op.bulk_push != 0 && static_cast<int>(gridDim.x) >= kMinHeraldLaunch + 1;
     const int herald_ctas = heralds ? mailbox_herald_ctas(push_ctas) : 0;
     PushSlot* const hand = reinterpret_cast<PushSlot*>(my_heap + cl.hand);
     const int cta = static_cast<int>(blockIdx.x);
     debug_delay(c, 4);
     if (cta < push_ctas) {
-      if (op.herald == 0) {
+      if (op.bulk_push == 0) {
         mailbox_push_rows<kProfile>(push, e, s_received, cta + (tid >> 5) * push_ctas, push_ctas * (kMailThreads / 32),
                                     reinterpret_cast<unsigned long long*>(dynamic_smem), lane, prof);
       } else if (tid < 32) {
@@ -1214,7 +1214,7 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
       hdr->cfin_count = 0;
       hdr->cwork_push = 0;
       hdr->cwork_reduce = 0;
-      if (kMode == kModeMailbox && op.herald != 0) {
+      if (kMode == kModeMailbox && op.bulk_push != 0) {
         PushSlot* hand = reinterpret_cast<PushSlot*>(my_heap + cl.hand);
         for (int i = 0; i < kMaxPushCtas; ++i) { hand[i].posted = 0; hand[i].final_rounds = 0; hand[i].heralded = 0; }
       }
@@ -1381,6 +1381,19 @@ cudaError_t combine_max_ctas(bool vec16, int fanout, int* ctas) {
 bool combine_can_mailbox(bool vec16, int fanout, int world, long long row_bytes) {
   // (A row travels as at most kPushStages pieces inside one round of a pusher.)
   return vec16 && fanout <= kPeerBatch && world > 1 && row_bytes <= static_cast<long long>(kPushStages) * kPushStageBytes;
+}
+
+// Whether the push CTAs of a mailbox launch move rows with bulk copies, fifteen per round, and let herald
+// CTAs publish them, or through registers, 48 rows per fence. Through registers the chain is shorter, but
+// no row is published before the 48 are complete: with rows above 8 KB that is 0.4 MB and more a time
+// (27 GB/s per SM either way), and the reducers wait. us of the kernel, ranks emulated on one GPU,
+// registers against bulk copies: 2048 wide, 8 x 240 and 4 x 480 tokens (1920 rows) 49 against 67 and 32
+// against 39; 7168 wide, 4 x 128 (32 rows per push CTA) 27 against 32, 2 x 480 (30) 24 against 29, 2 x 900
+// (56) 44.9 against 42.7, 4 x 256 (64) 50 against 42, 4 x 480 (120) 85 against 65; 16384 wide, 3 x 512
+// (73) 120 against 87. Above 1920 rows the register push has not been tried.
+bool combine_bulk_push(int slot_capacity, long long row_bytes, int ctas) {
+  if (slot_capacity > 1920) return true;
+  return row_bytes > 8192 && slot_capacity > 40 * mailbox_push_ctas(ctas);
 }
 
 cudaError_t launch_combine(const CombineArgs& args, int ranks, int ctas_per_rank, bool vec16, int fanout,

@@ -244,7 +244,8 @@ struct CombineOp {
   int segments;
   int vec16;
   int partial_rows;       // rows of `partial`; fewer than the received rows is an error
-  int herald;             // mailbox protocol: non-zero = arrival words are published by herald CTAs (large batches)
+  int bulk_push;          // mailbox protocol: non-zero = push CTAs move rows with bulk copies and herald CTAs publish
+                          // their arrival words; zero = through registers, published by the push CTA itself
 };
 
 // Bounded timing record of operations that run from CUDA graphs (every replay is a new
