@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
   __shared__ int s_base, s_total, s_dirty, s_counted;
   __shared__ unsigned long long s_full[kLoneMovers * kLoneStages];
 
-  launch_dependents();
+  launch_dependents();                    // ahead of everything: right only because this kernel is launched plainly
   const unsigned g = ld_volatile_u32(&hdr->disp_epoch) + 1;
 
   // ---- movers: warp w takes pieces w, w + kLoneMovers, ... of the CTA's rows ----------------

@@ -336,7 +336,9 @@ __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontr
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Programmatic dependent launch: the kernel's dispatch and prologue overlap the tail of the kernel
 // before it on the stream. Kernels launched this way call wait_for_previous before they touch data,
-// and launch_dependents only after that, so a kernel that runs knows every earlier one is complete.
+// and launch_dependents only after that, so a kernel that runs knows every earlier one is complete. A
+// kernel that is only ever launched plainly starts behind everything before it and may call
+// launch_dependents at once (dispatch_lone_kernel); launched with this function, it would break the rule.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_chained(void (*kernel)(Params...), int ctas, int threads, int cluster, size_t smem,
                            cudaStream_t stream, Args... args) {

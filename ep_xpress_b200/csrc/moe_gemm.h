@@ -49,6 +49,10 @@ cudaError_t launch_moe_scatter(const void* hidden, const int* entry_pos, const i
 // that was given to the align step. With `gather_rows` (= the align step's sorted_row), `sorted_x`
 // is the UNSORTED activation matrix [gather_height, hidden]: the kernel's TMA producer gathers the
 // rows of every tile itself (four rows per copy) and no scatter launch or sorted copy is needed.
+// Order: without `gather_rows` both GEMMs read `counters` and `tiles` BEFORE they wait for the kernel
+// launched before them on the stream. A launch that itself waits for the align step therefore has to
+// stand between it and them (the scatter; for the second GEMM, the first); right behind the align step
+// they would read a half-written list.
 cudaError_t launch_moe_gemm_gate_up(const void* sorted_x, const void* w13, void* act, const int* counters,
                                     const int* tiles, int* error_flag, long long rows, long long max_sorted_rows,
                                     int experts, int hidden_size, int inter_size, int sms, cudaStream_t stream,
