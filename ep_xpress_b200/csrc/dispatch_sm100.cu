@@ -922,6 +922,9 @@ __global__ void __launch_bounds__(kThreads, 1) dispatch_lone_kernel(const __grid
         }
         if (++stage == kLoneStages) stage = 0;
       }
+      // After giving up: the loads still under way target this CTA's shared memory.
+      for (int s = 0; s < kLoneStages && loading != 0u; ++s)
+        if ((loading >> s) & 1u) mbarrier_wait_bounded(full + s, (parity >> s) & 1u, c.timeout_ns);
       bulk_wait_all_complete();
     }
   } else {
