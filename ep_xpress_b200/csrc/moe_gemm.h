@@ -18,7 +18,7 @@ constexpr int kMoeGateUpTile = 128;   // intermediate columns produced by one GE
 constexpr int kMoeDownTile = 256;     // hidden columns produced by one GEMM-2 tile
 
 struct MoeSizes {
-  long long max_sorted_rows;   // workspace rows: every local pair plus one tile of slack per expert
+  long long max_sorted_rows;   // workspace rows: every local pair, and up to experts + 1 tiles of slack that no kernel needs
   int max_tiles;               // the same in tiles of `tile_rows`
 };
 

@@ -33,7 +33,7 @@ class GroupedSwiGLU:
         (measured at hidden 7168 / inter 2048, 2 GPUs, 4096 tokens per rank: 7.4 ms against
         3.7 ms with a copy kernel, whose cost is 0.1 to 0.15 ms).
 
-        ``pair_ctas`` is accepted either way: every GEMM runs on clusters of two CTAs.
+        ``pair_ctas`` is accepted and changes nothing: every GEMM runs on clusters of two CTAs.
 
         The default is the worst case (every slot of every row is local). A tighter,
         CPU-known bound saves workspace; exceeding it is reported by :meth:`check`,
@@ -50,8 +50,8 @@ class GroupedSwiGLU:
         self.native = _native_loader.load()
         self.w13, self.w2 = w13.contiguous(), w2.contiguous()
         self.experts, self.hidden, self.inter, self.topk, self.max_rows = experts, hidden, inter, topk, max_rows
-        self.pair_ctas = bool(pair_ctas)        # accepted either way: the GEMMs always run on clusters of two CTAs
-        tile = self.native.MOE_TILE_ROWS * (2 if self.pair_ctas else 1)
+        self.pair_ctas = bool(pair_ctas)        # accepted, without effect
+        tile = self.native.MOE_TILE_ROWS
         worst_rows, _ = self.native.moe_sizes(max_rows, topk, experts, tile)
         if max_local_pairs is None:
             sorted_rows = worst_rows

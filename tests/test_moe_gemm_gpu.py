@@ -61,16 +61,15 @@ def test_matches_fp32_reference(rows, topk, experts, hidden, inter, valid, gathe
     assert torch.equal(again[:valid], out[:valid])
 
 
-@pytest.mark.parametrize("pair_ctas", [False, True])
-def test_benchmarked_shape_matches_fp32_reference(pair_ctas):
+def test_benchmarked_shape_matches_fp32_reference():
     """Hidden 7168, intermediate 2048 (112 k-steps, 16 and 28 column tiles): the shape of the layer
-    benchmark, on a few experts and a few hundred rows, both kernels, gathered and pre-gathered
-    activations bit-identical to each other."""
+    benchmark, on a few experts and a few hundred rows, gathered and pre-gathered activations
+    bit-identical to each other."""
     rows, topk, experts, hidden, inter, valid = 520, 8, 4, 7168, 2048, 500
     x, ids, weights, count, w13, w2 = make_case(rows, topk, experts, hidden, inter, valid, seed=11, local_fraction=0.4)
     outs = []
     for gather_loads in (True, False):
-        runner = GroupedSwiGLU(w13, w2, max_rows=rows, topk=topk, pair_ctas=pair_ctas, gather_loads=gather_loads)
+        runner = GroupedSwiGLU(w13, w2, max_rows=rows, topk=topk, gather_loads=gather_loads)
         out = torch.full((rows, hidden), 7.0, dtype=torch.bfloat16, device="cuda")
         runner(x, ids, weights, count, out=out)
         runner.check()
@@ -81,25 +80,29 @@ def test_benchmarked_shape_matches_fp32_reference(pair_ctas):
     assert (outs[0][valid:] == 7.0).all()
 
 
-@pytest.mark.parametrize("rows,topk,experts,hidden,inter,valid", [
-    (64, 2, 2, 256, 128, 64),
-    (700, 4, 3, 512, 256, 650),
-    (1000, 8, 8, 1024, 384, 1000),
+@pytest.mark.parametrize("valid,topk,experts,hidden,inter", [
+    (16, 2, 2, 256, 128),
+    (100, 4, 3, 512, 256),
+    (250, 8, 8, 1024, 384),
+    (650, 4, 3, 512, 256),
 ])
-def test_cta_pairs_match_fp32_reference_and_single_cta_path(rows, topk, experts, hidden, inter, valid):
-    """tcgen05 cta_group::2 on clusters of two CTAs (256-row tiles) against the same oracle."""
-    x, ids, weights, count, w13, w2 = make_case(rows, topk, experts, hidden, inter, valid, seed=rows + 1)
-    pair = GroupedSwiGLU(w13, w2, max_rows=rows, topk=topk, pair_ctas=True)
-    out = torch.full((rows, hidden), 7.0, dtype=torch.bfloat16, device="cuda")
-    pair(x, ids, weights, count, out=out)
-    pair.check()
+def test_padding_of_the_batch_does_not_change_its_rows(valid, topk, experts, hidden, inter):
+    """The number of rows a batch is padded to bounds the token tiles: other tile widths, ring depths and
+    numbers of epilogue warps, the same sums. ``pair_ctas`` is accepted and changes nothing."""
+    x, ids, weights, count, w13, w2 = make_case(valid, topk, experts, hidden, inter, valid, seed=valid + 1)
     want = swiglu_reference(x, ids, weights, valid, w13, w2)
-    assert_elementwise_close(out[:valid], want[:valid])
-    assert (out[valid:] == 7.0).all()
-    single = GroupedSwiGLU(w13, w2, max_rows=rows, topk=topk)
-    other = torch.empty_like(out)
-    single(x, ids, weights, count, out=other)
-    assert torch.equal(other[:valid], out[:valid])     # same accumulation order per output row
+    first = None
+    for rows, pair_ctas in ((valid, False), (valid, True), (2 * valid, False), (1300, True)):
+        padded = [torch.cat([t, torch.full((rows - valid, t.shape[1]), fill, dtype=t.dtype, device=t.device)])
+                  for t, fill in ((x, 0), (ids, -1), (weights, 0))]
+        runner = GroupedSwiGLU(w13, w2, max_rows=rows, topk=topk, pair_ctas=pair_ctas)
+        out = torch.full((rows, hidden), 7.0, dtype=torch.bfloat16, device="cuda")
+        runner(*padded, count, out=out)
+        runner.check()
+        assert (out[valid:] == 7.0).all()
+        first = out if first is None else first
+        assert torch.equal(out[:valid].view(torch.int16), first[:valid].view(torch.int16))
+    assert_elementwise_close(first[:valid], want[:valid])
 
 
 @pytest.mark.parametrize("counts,pad", [
