@@ -92,7 +92,7 @@ class Slot:
     busy: bool = False                 # dispatched, combine not yet enqueued
     released: bool = False
     tag: object = field(default=None, repr=False)
-    cut: object = field(default=None, repr=False)   # internal views of a pool slot at the shape it was last used with
+    cut: object = field(default=None, repr=False)   # views of a pool slot at the shape it was last used with, never handed out
     bases: Optional[List[int]] = None  # allocation start per local rank when guard bands surround the slot
     guards: Optional[List[torch.Tensor]] = None   # uint8 views of the guard bands (diagnostics)
 
