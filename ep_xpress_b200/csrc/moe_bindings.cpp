@@ -64,8 +64,10 @@ void moe_forward(const at::Tensor& hidden, const at::Tensor& local_ids, const at
   TORCH_CHECK(tiles.numel() >= 4 * moe_token_tiles(sorted_rows, static_cast<int>(experts)), "the tile list is too small");
   TORCH_CHECK((gathered || sorted_x.numel() >= sorted_rows * hidden_size) && y.numel() >= sorted_rows * hidden_size &&
               act.numel() >= sorted_rows * inter, "workspace tensors are too small");
-  TORCH_CHECK(!gathered || (reinterpret_cast<uintptr_t>(hidden.data_ptr()) % 16 == 0 && rows > 0),
-              "gathered loads need a 16-byte aligned, non-empty activation matrix");
+  // The row movers use 16-byte accesses: a misaligned view would fault on the GPU.
+  TORCH_CHECK(rows == 0 || (reinterpret_cast<uintptr_t>(hidden.data_ptr()) % 16 == 0 &&
+              reinterpret_cast<uintptr_t>(partial.data_ptr()) % 16 == 0), "hidden and partial must be 16-byte aligned");
+  TORCH_CHECK(!gathered || rows > 0, "gathered loads need a non-empty activation matrix");
   c10::cuda::CUDAGuard guard(hidden.device());
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_handle);
   const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;

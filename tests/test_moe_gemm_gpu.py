@@ -146,6 +146,15 @@ def test_negative_count_is_an_empty_batch(rows, gather_loads, count):
     assert (out == 7.0).all() and runner.counters.tolist() == [0, 0]
 
 
+def test_misaligned_rows_are_rejected_on_the_host():
+    x, ids, weights, count, w13, w2 = make_case(64, 2, 2, 256, 128, 64, seed=6)
+    runner = GroupedSwiGLU(w13, w2, max_rows=64, topk=2)
+    skewed = torch.zeros(64 * 256 + 1, dtype=torch.bfloat16, device="cuda")[1:].view(64, 256)
+    for hidden, out in ((skewed, torch.empty_like(x)), (x, skewed)):
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            runner(hidden, ids, weights, count, out=out)
+
+
 def test_pair_bound_overflow_is_reported():
     x, ids, weights, count, w13, w2 = make_case(512, 4, 2, 256, 128, 512, seed=3, local_fraction=1.0)
     runner = GroupedSwiGLU(w13, w2, max_rows=512, topk=4, max_local_pairs=128)
