@@ -235,9 +235,10 @@ constexpr int kPushStageBytes = 14336;
 constexpr size_t kMailSmemBytes = static_cast<size_t>(kPushStages) * kPushStageBytes;
 
 // Push CTAs of a mailbox launch of `ctas` CTAs (at least two): enough SMs to keep the link
-// busy - a pusher moves fifteen rows per round trip - and the rest reduce, which is the heavier
-// job in bytes (every pushed row is read again, plus the local rows and the output). With
-// heralds, one CTA per sixteen pushers is taken from the reducers.
+// busy, and the rest reduce, which is the heavier job in bytes (every pushed row is read again,
+// plus the local rows and the output). With heralds, one CTA per sixteen pushers is taken from
+// the reducers. The share dates from the stage-ring reduce and was not swept with the present
+// reducers; at 4 x 1024 x 7168, top-8, the pushers end 12 us before the reducers do (105 of 118).
 __host__ __device__ __forceinline__ int mailbox_push_ctas(int ctas) {
   const int wanted = ctas * 7 / 16;
   return wanted < 1 ? 1 : (wanted > kMaxPushCtas ? kMaxPushCtas : wanted);
@@ -245,6 +246,19 @@ __host__ __device__ __forceinline__ int mailbox_push_ctas(int ctas) {
 constexpr int kHeraldWarpsPerCta = 16;
 __host__ __device__ __forceinline__ int mailbox_herald_ctas(int push_ctas) {
   return (push_ctas + kHeraldWarpsPerCta - 1) / kHeraldWarpsPerCta;
+}
+// Whether the push CTAs move rows with bulk copies, fifteen per round, and let herald CTAs publish them, or
+// through registers, two rows of every warp per fence. (It concerns this rank only: peers see the same
+// rows and arrival words either way.) Through registers the chain is shorter, but no row is published
+// before all of a fence are complete. With rows above 8 KB and most warps on their second that is half a
+// MB a time (27 GB/s per SM either way), and the reducers wait. us of the kernel, ranks emulated on one
+// GPU, registers against bulk copies, remote rows per push CTA in brackets: 7168 wide, 2 x 480 tokens (15)
+// 24 against 29, 4 x 128 (22) 27 against 32, 2 x 900 (28) 45 against 42, 8 x 48 (32) 35 against 39, 4 x 256
+// (43) 48 against 43, 8 x 100 (66) 67 against 54, 4 x 480 (81) 85 against 65; 16384 wide, 3 x 512 (48) 120 against 87; 2048 wide, 8 x 240 (160) and 4 x 480
+// (81) 49 against 67 and 32 against 39. Slots above 1920 rows have not been tried with registers.
+constexpr int kRegisterPushRows = 1920;
+__device__ __forceinline__ bool mailbox_bulk_push(int slot_capacity, long long row_bytes, int remote_rows, int push_ctas) {
+  return slot_capacity > kRegisterPushRows || (row_bytes > 8192 && remote_rows > kMailThreads / 32 * 3 / 2 * push_ctas);
 }
 // Smallest launch that has a push CTA, its herald CTA and a reduce CTA.
 constexpr int kMinHeraldLaunch = 3;
@@ -1050,17 +1064,19 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
   reduce.single_round = single_round; reduce.timeout_ns = c.timeout_ns; reduce.profile = op.profile;
   reduce.cta = static_cast<int>(blockIdx.x);
   reduce.ctas = static_cast<int>(gridDim.x);
+  const int push_ctas = mailbox_push_ctas(static_cast<int>(gridDim.x));
+  const bool bulk_push = kMode == kModeMailbox &&
+                         mailbox_bulk_push(op.slot_capacity, row_bytes, s_received - s_rows_from[self], push_ctas);
   if (kMode == kModeMailbox) {
     // ---- push CTAs, herald CTAs and reduce CTAs side by side ----
     // (A mailbox launch has at least two CTAs; heralds are used from kMinHeraldLaunch CTAs on.)
-    const int push_ctas = mailbox_push_ctas(static_cast<int>(gridDim.x));
-    const bool heralds = op.bulk_push != 0 && static_cast<int>(gridDim.x) >= kMinHeraldLaunch + 1;
+    const bool heralds = bulk_push && static_cast<int>(gridDim.x) >= kMinHeraldLaunch + 1;
     const int herald_ctas = heralds ? mailbox_herald_ctas(push_ctas) : 0;
     PushSlot* const hand = reinterpret_cast<PushSlot*>(my_heap + cl.hand);
     const int cta = static_cast<int>(blockIdx.x);
     debug_delay(c, 4);
     if (cta < push_ctas) {
-      if (op.bulk_push == 0) {
+      if (!bulk_push) {
         mailbox_push_rows<kProfile>(push, e, s_received, cta + (tid >> 5) * push_ctas, push_ctas * (kMailThreads / 32),
                                     reinterpret_cast<unsigned long long*>(dynamic_smem), lane, prof);
       } else if (tid < 32) {
@@ -1214,7 +1230,7 @@ __device__ __forceinline__ void combine_body(const CombineOp& op, char* dynamic_
       hdr->cfin_count = 0;
       hdr->cwork_push = 0;
       hdr->cwork_reduce = 0;
-      if (kMode == kModeMailbox && op.bulk_push != 0) {
+      if (bulk_push) {
         PushSlot* hand = reinterpret_cast<PushSlot*>(my_heap + cl.hand);
         for (int i = 0; i < kMaxPushCtas; ++i) { hand[i].posted = 0; hand[i].final_rounds = 0; hand[i].heralded = 0; }
       }
@@ -1381,19 +1397,6 @@ cudaError_t combine_max_ctas(bool vec16, int fanout, int* ctas) {
 bool combine_can_mailbox(bool vec16, int fanout, int world, long long row_bytes) {
   // (A row travels as at most kPushStages pieces inside one round of a pusher.)
   return vec16 && fanout <= kPeerBatch && world > 1 && row_bytes <= static_cast<long long>(kPushStages) * kPushStageBytes;
-}
-
-// Whether the push CTAs of a mailbox launch move rows with bulk copies, fifteen per round, and let herald
-// CTAs publish them, or through registers, 48 rows per fence. Through registers the chain is shorter, but
-// no row is published before the 48 are complete: with rows above 8 KB that is 0.4 MB and more a time
-// (27 GB/s per SM either way), and the reducers wait. us of the kernel, ranks emulated on one GPU,
-// registers against bulk copies: 2048 wide, 8 x 240 and 4 x 480 tokens (1920 rows) 49 against 67 and 32
-// against 39; 7168 wide, 4 x 128 (32 rows per push CTA) 27 against 32, 2 x 480 (30) 24 against 29, 2 x 900
-// (56) 44.9 against 42.7, 4 x 256 (64) 50 against 42, 4 x 480 (120) 85 against 65; 16384 wide, 3 x 512
-// (73) 120 against 87. Above 1920 rows the register push has not been tried.
-bool combine_bulk_push(int slot_capacity, long long row_bytes, int ctas) {
-  if (slot_capacity > 1920) return true;
-  return row_bytes > 8192 && slot_capacity > 40 * mailbox_push_ctas(ctas);
 }
 
 cudaError_t launch_combine(const CombineArgs& args, int ranks, int ctas_per_rank, bool vec16, int fanout,

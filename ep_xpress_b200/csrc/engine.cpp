@@ -289,7 +289,6 @@ class Engine {
     for (size_t i = 0; i < n; ++i) {
       args.op[i].segments = segments;
       args.op[i].vec16 = vec16 ? 1 : 0;
-      args.op[i].bulk_push = combine_bulk_push(static_cast<int>(slot_capacity[i]), static_cast<long long>(hidden_) * 2, ctas) ? 1 : 0;
     }
     attach_profile(profile, ctas, n, [&](size_t i, unsigned long long* p) { args.op[i].profile = p; });
     attach_samples(samples, n, [&](size_t i, unsigned long long* ring, int capacity) {

@@ -31,9 +31,6 @@ cudaError_t launch_dispatch(const DispatchArgs& args, int ranks, const RankCtx& 
 // up to eight, rows of up to 112 KiB and groups of two or more ranks (`combine_can_mailbox`); elsewhere, and when not
 // asked for, the sequential protocol runs. All ranks of a group must choose the same protocol.
 bool combine_can_mailbox(bool vec16, int fanout, int world, long long row_bytes);
-// CombineOp::bulk_push of a mailbox launch of `ctas` CTAs per rank over a slot of `slot_capacity` rows.
-// (It concerns this rank only: peers see the same rows and arrival words either way.)
-bool combine_bulk_push(int slot_capacity, long long row_bytes, int ctas);
 cudaError_t launch_combine(const CombineArgs& args, int ranks, int ctas_per_rank, bool vec16, int fanout,
                            const RankCtx& host_ctx, bool mailbox, bool cooperative, cudaStream_t stream);
 

@@ -140,11 +140,11 @@ struct SlotLayout {
 };
 
 // Words 8.. of a CTA's profile record (profiling launches only). Words 0..7 are phase stamps
-// on the GPU's global timer (combine: 4..7 hold pipeline cycle counts instead).
+// on the GPU's global timer (combine: 4..7 hold cycle counts of the stage rings instead, zero in mailbox launches).
 enum ProfileWord : int {
   kProfRows = 8,          // rows this CTA stored to destination planes (dispatch) or pushed (combine)
   kProfBytes = 9,         // payload bytes of those rows
-  kProfItems = 10,        // combine: (token, row segment) items this CTA's producers issued
+  kProfItems = 10,        // combine: (token, row segment) items this CTA reduced
   kProfPolls = 11,        // iterations of bounded waits on words that peers write
   kProfFirstPublish = 12, // time of this CTA's first publication to a peer (0: none)
   kProfFirstReceive = 13, // time this CTA first saw data or a word from a peer (0: none)
@@ -152,7 +152,7 @@ enum ProfileWord : int {
   kProfCompletion = 15,   // index of the last phase stamp the CTA wrote
   kProfMode = 16,         // combine: 1 + protocol (0 register, 1 bulk, 2 mailbox); dispatch: 1 register path, 2 bulk-copy movers
   kProfPushWait = 17,     // combine, mailbox: ns the CTA's pushers spent waiting for their copies (loads landed, stores completed)
-  kProfArrivalWait = 18,  // combine, mailbox: ns producer 0 spent waiting for arrival words of peers' rows
+  kProfArrivalWait = 18,  // combine, mailbox: ns the lanes of warp 0 spent waiting for arrival words of peers' rows
   kProfStoreCycles = 19,  // combine, bulk-copy reduce: cycles consumer warp 0 spent converting and storing finished chunks
 };
 
@@ -244,8 +244,6 @@ struct CombineOp {
   int segments;
   int vec16;
   int partial_rows;       // rows of `partial`; fewer than the received rows is an error
-  int bulk_push;          // mailbox protocol: non-zero = push CTAs move rows with bulk copies and herald CTAs publish
-                          // their arrival words; zero = through registers, published by the push CTA itself
 };
 
 // Bounded timing record of operations that run from CUDA graphs (every replay is a new

@@ -305,7 +305,7 @@ def test_both_combine_protocols_match_the_oracle(world, hidden, topk, tokens, ct
     (3, 512, 3, 641, None),                   # the smallest with heralds: 21 pushers, a full and a partial herald CTA
     (2, 64, 2, 2000, 74),                     # two full herald CTAs, several rounds per pusher
     (2, 256, 2, 1000, 4), (2, 256, 2, 1000, 3),   # the smallest launch with a herald CTA; pushers that publish themselves
-    (4, 4104, 4, 160, 37), (4, 4104, 4, 161, 37),   # rows above 8 KB: 40 per push CTA, and more
+    (2, 4104, 4, 108, 7), (2, 4104, 4, 109, 7),   # rows above 8 KB: 36 per push CTA (108 remote rows), and one more
 ])
 def test_arrival_words_leave_through_one_warp(world, hidden, topk, tokens, ctas):
     """Who fences and stores the arrival words, at the sizes where that changes; with and without delays."""
