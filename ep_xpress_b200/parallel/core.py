@@ -192,14 +192,16 @@ class TransportCore:
         return max(1, min(budget, wanted))
 
     def pick_combine_ctas(self, tokens: int, capacity: int, budget: Optional[int] = None) -> int:
-        """CTAs per rank of a combine. Under the mailbox protocol 7/16 of them (at most 64) only
-        push - fifteen received rows per round trip each - and the others reduce four (token, row
-        segment) items at a time; small batches get enough CTAs for one round trip to move
-        everything (one round per pusher also for the tiniest batch), and never fewer than two (one
-        pushes, one reduces)."""
+        """CTAs per rank of a combine. Under the mailbox protocol 7/16 of them (at most 64) only push and
+        the others reduce, one (token, row segment) item per warp. One CTA per token or per six rows of
+        capacity, and never fewer than two (one pushes, one reduces). More CTAs than that only take SMs
+        from others: us of the kernel at 2 x 64 / 4 x 32 / 8 x 16 tokens by CTAs per rank, hidden 7168 /
+        7168 / 2048: with 18, 14.8 / 17.7 / 12.2; with 37, 11.9 / 13.2 / -; with 64, 11.6 / - / -."""
         budget = self.max_ctas if budget is None else max(1, min(budget, self.max_ctas))
-        # The pushers walk the received rows interleaved over the peers in blocks of eight, holes
-        # included: even one row per peer is (world - 1) * 8 work items, fifteen per pusher round.
+        # Tiny batches of wide groups: a token's rows come from many peers, and two CTAs serialise them
+        # (one token per rank, hidden 7168, us with 2 / 3 / 10 CTAs: 8 ranks 14.4 / 13.0 / 11.7, 4 ranks
+        # 10.1 / 10.0 / 10.9). The floor is what the bulk-copy pushers need for one round: fifteen items
+        # each of an order that interleaves the peers in blocks of eight, holes included.
         peers = max(getattr(self, "world", 1) - 1, 0)
         pushers = -(-peers * 8 // 15)
         floor = max(2, -(-pushers * 16 // 7))

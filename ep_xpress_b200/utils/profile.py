@@ -14,12 +14,12 @@ One record per CTA (times in ns on the GPU's global timer):
 * words 0..7: phase stamps. Dispatch: start, routed, barrier, counts_in, payload_done,
   signalled, padded, done. Combine: start, published (sequential protocol: this CTA's rows are
   out; mailbox protocol: its first pusher is done), peers_ready (sequential: every peer has
-  signalled; mailbox: pushers and reducers have joined), reduced; words 4..7 hold pipeline
-  cycle counts of the combine's first reduce pipeline instead.
-* rows / bytes the CTA stored to other planes, (token, segment) items its reducers issued,
+  signalled; mailbox: pushers and reducers have joined), reduced; words 4..7 hold cycle counts of
+  the first stage-ring pipeline instead (sequential protocol; zero in mailbox launches).
+* rows / bytes the CTA stored to other planes, (token, segment) items it reduced,
   poll iterations of its bounded waits, the times of its first publication to a peer and of
   the first peer word it saw, the rank's status and the last stamp it reached, the protocol
-  it ran, and how long its pushers / its first producer waited.
+  it ran, and how long its pushers / its first reducing warp waited.
 
 The report derives DISJOINT per-CTA phases from consecutive stamps; by construction they sum
 to the CTA's elapsed time, which :func:`check_invariants` verifies together with the
